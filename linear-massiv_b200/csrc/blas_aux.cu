@@ -113,85 +113,6 @@ __global__ void __launch_bounds__(kSwapThreads) laswp_kernel(T* A, long long lda
     if (active) A[(long long)list_r[i] * lda + col] = stage[i * 32 + lane];
 }
 
-// The same interchanges split in two launches for wide matrices: one CTA
-// composes the swaps ipiv[k0..k1) into the list of (row, source row) pairs
-// that change (plan[0] = count, then rows, then sources, 2 * kSwapChunk
-// each), so that the column blocks need no serial prologue of their own.
-// Every touched row (the swap positions k0..k1-1 and the distinct pivot rows
-// outside them) is a thread, which finds its source by walking the swap list
-// backwards: source(r) = tau_k0(tau_k0+1(... tau_k1-1(r))).
-__global__ void __launch_bounds__(2 * kSwapChunk) swap_plan_kernel(int nrows, const int* __restrict__ ipiv, int k0,
-                                                                   int k1, int* plan, int* status) {
-  __shared__ int piv[kSwapChunk];
-  __shared__ int mm_sh;
-  const int tid = threadIdx.x;
-  const int cnt = k1 - k0;
-  if (tid < cnt) {
-    int p = __ldg(ipiv + k0 + tid);
-    if (p < 0 || p >= nrows) {  // a bad swap list: record it, treat as no swap
-      atomicCAS(status, 0, LM_DEVERR_BOUNDS);
-      p = k0 + tid;
-    }
-    piv[tid] = p;
-  }
-  if (tid == 0) mm_sh = 0;
-  __syncthreads();
-  int r = -1;
-  if (tid < cnt) {
-    r = k0 + tid;
-  } else if (tid < 2 * cnt) {
-    const int q = tid - cnt;
-    const int p = piv[q];
-    bool first = p < k0 || p >= k1;  // swap positions are covered above
-    for (int e = 0; e < q && first; ++e) first = piv[e] != p;
-    if (first) r = p;
-  }
-  if (r >= 0) {
-    int x = r;
-    for (int q = cnt - 1; q >= 0; --q) {
-      const int k = k0 + q, p = piv[q];
-      x = (x == k) ? p : ((x == p) ? k : x);
-    }
-    if (x != r) {
-      const int at = atomicAdd(&mm_sh, 1);
-      plan[1 + at] = r;
-      plan[1 + 2 * kSwapChunk + at] = x;
-    }
-  }
-  __syncthreads();
-  if (tid == 0) plan[0] = mm_sh;
-}
-
-// Gather every changing row's source over a 32-column block into shared
-// memory, then scatter (the plan of swap_plan_kernel).
-template <typename T>
-__global__ void __launch_bounds__(kSwapThreads) swap_apply_kernel(T* A, long long lda, const int* __restrict__ plan,
-                                                                  int ca0, int ca1, int cb0, int cb1) {
-  __shared__ int list_r[2 * kSwapChunk];
-  __shared__ int list_s[2 * kSwapChunk];
-  extern __shared__ __align__(16) unsigned char sm[];
-  T* stage = reinterpret_cast<T*>(sm);  // [2 * kSwapChunk][32]
-  const int tid = threadIdx.x;
-  const int mm = __ldg(plan);
-  for (int i = tid; i < mm; i += kSwapThreads) {
-    list_r[i] = __ldg(plan + 1 + i);
-    list_s[i] = __ldg(plan + 1 + 2 * kSwapChunk + i);
-  }
-  __syncthreads();
-  const int na = ca1 - ca0, ncols = na + (cb1 - cb0);
-  const int lane = tid & 31, warp = tid >> 5;
-  const int t = blockIdx.x * 32 + lane;
-  const bool active = t < ncols;
-  const int col = t < na ? ca0 + t : cb0 + (t - na);
-#pragma unroll 8
-  for (int i = warp; i < mm; i += kSwapThreads / 32)
-    if (active) stage[i * 32 + lane] = A[(long long)list_s[i] * lda + col];
-  __syncthreads();
-#pragma unroll 8
-  for (int i = warp; i < mm; i += kSwapThreads / 32)
-    if (active) A[(long long)list_r[i] * lda + col] = stage[i * 32 + lane];
-}
-
 // All interchanges ipiv[0..n) on a narrow block B (n x nrhs) at once:
 // W(i, :) = B(sigma(i), :) with sigma(i) = tau_0(tau_1(... tau_{n-1}(i))),
 // tau_k the transposition (k, ipiv[k]).  Thread i walks the swap list
@@ -421,7 +342,7 @@ int grid_for(long long total, int threads, int sms) {
 
 template <typename T>
 int laswp(T* A, long long lda, int nrows, const int* ipiv, int k0, int k1, int ca0, int ca1, int cb0, int cb1,
-          int* status, cudaStream_t st, int* plan) {
+          int* status, cudaStream_t st) {
   ca1 = std::max(ca0, ca1);
   cb1 = std::max(cb0, cb1);
   const int cols = (ca1 - ca0) + (cb1 - cb0);
@@ -432,22 +353,12 @@ int laswp(T* A, long long lda, int nrows, const int* ipiv, int k0, int k1, int c
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
     LM_CUDA_TRY(cudaFuncSetAttribute(laswp_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    LM_CUDA_TRY(cudaFuncSetAttribute(swap_apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set[dev] = true;
   }
-  // wide: plan once, then the column blocks; narrow: one self-contained launch
-  const bool planned = plan != nullptr && cols > 4 * 32;
   for (int s0 = k0; s0 < k1; s0 += kSwapChunk) {
     const int s1 = std::min(k1, s0 + kSwapChunk);
-    if (planned) {
-      swap_plan_kernel<<<1, 2 * kSwapChunk, 0, st>>>(nrows, ipiv, s0, s1, plan, status);
-      swap_apply_kernel<T><<<cdiv(cols, 32), kSwapThreads, smem, st>>>(A, lda, plan, ca0, ca1, cb0, cb1);
-      count_launch(2);
-    } else {
-      laswp_kernel<T><<<cdiv(cols, 32), kSwapThreads, smem, st>>>(A, lda, nrows, ipiv, s0, s1, ca0, ca1, cb0, cb1,
-                                                                  status);
-      count_launch(1);
-    }
+    laswp_kernel<T><<<cdiv(cols, 32), kSwapThreads, smem, st>>>(A, lda, nrows, ipiv, s0, s1, ca0, ca1, cb0, cb1, status);
+    count_launch(1);
     LM_CUDA_TRY(cudaGetLastError());
   }
   return LM_OK;
@@ -563,9 +474,8 @@ int dresidual(Ctx& c, int n, int nrhs, const double* A, long long lda, const dou
   return dgemm(c, d, st);
 }
 
-template int laswp<double>(double*, long long, int, const int*, int, int, int, int, int, int, int*, cudaStream_t,
-                           int*);
-template int laswp<float>(float*, long long, int, const int*, int, int, int, int, int, int, int*, cudaStream_t, int*);
+template int laswp<double>(double*, long long, int, const int*, int, int, int, int, int, int, int*, cudaStream_t);
+template int laswp<float>(float*, long long, int, const int*, int, int, int, int, int, int, int*, cudaStream_t);
 template int laswp_narrow<double>(double*, long long, int, int, const int*, double*, int*, cudaStream_t);
 template int laswp_narrow<float>(float*, long long, int, int, const int*, float*, int*, cudaStream_t);
 template int laswp_perm<double>(double*, long long, int, int, const int*, double*, cudaStream_t);

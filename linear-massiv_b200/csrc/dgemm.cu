@@ -81,7 +81,7 @@ struct GemmCfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   // C staged in smem as BN / 16 boxes of BM x 16 doubles (128-byte swizzle)
   static constexpr int C_BYTES = CSM ? BM * BN * 8 : 0;
-  static constexpr int BUDGET = CSM ? 227 * 1024 - C_BYTES - 2048 : (200 * 1024) / MINB;
+  static constexpr int BUDGET = CSM ? (227 * 1024 - 2048) / MINB - C_BYTES : (200 * 1024) / MINB;
   static constexpr int STAGES = BUDGET / STAGE_BYTES > 8 ? 8 : BUDGET / STAGE_BYTES;
   static constexpr int SMEM = STAGES * STAGE_BYTES + C_BYTES + 2 * STAGES * 8 + 16 + 1024;  // + alignment slack
   static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
@@ -444,6 +444,14 @@ int dgemm(Ctx& ctx, const GemmDesc& d, cudaStream_t st) {
   Prof prof(ctx, kPhaseGemm, flops, bytes, st);
   const bool narrow = (d.n <= 64 || d.k <= 256) && !d.lower_only;
   const bool c_tma = d.beta != 0.0 && !(reinterpret_cast<uintptr_t>(d.C) & 15) && !(d.ldc & 1);
+  const int sms = d.max_sms > 0 ? std::min(d.max_sms, ctx_num_sms(ctx)) : ctx_num_sms(ctx);
+  if (d.k <= 256 && d.n > 64 && c_tma && !d.lower_only && cdiv(d.m, 128) * cdiv(d.n, 128) < sms) {
+    // not one 128 x 128 tile per SM (a panel's own columns, the end of a
+    // factorisation): a quarter of the tile in about half the time
+    if (d.a_trans) return launch_dmma<64, 64, true, false, 2, true>(ctx, d, st);
+    if (d.b_trans) return launch_dmma<64, 64, false, true, 2, true>(ctx, d, st);
+    return launch_dmma<64, 64, false, false, 2, true>(ctx, d, st);
+  }
   if (d.k <= 256 && d.n > 64 && c_tma) {
     int rc;
     if (d.a_trans)

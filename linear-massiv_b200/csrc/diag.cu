@@ -518,7 +518,5 @@ int nopiv_diag(float* A11, long long lda, int w, int base, float* Lhi, float* Ll
 
 template int tri_inv_lower<double>(const double*, long long, int, bool, double*, long long, double*, cudaStream_t);
 template int trsm_lower_small<double>(const double*, long long, int, bool, double*, long long, int, cudaStream_t);
-template int trsm_lower_small<float>(const float*, long long, int, bool, float*, long long, int, cudaStream_t);
-template int tri_inv_lower<float>(const float*, long long, int, bool, float*, long long, float*, cudaStream_t);
 
 }  // namespace lm

@@ -2,17 +2,12 @@
 //
 // dgetrf — right-looking blocked LU, outer panels of kNB = 128 columns so the
 //   trailing update is a k = 128 DMMA GEMM (compute-bound on B200, unlike the
-//   reference's k = 32 update, LU.hs:311-357).  Each 128-wide panel is
-//   factored recursively (halves down to a cluster leaf of <= 32 columns):
-//     left half -> swap right half -> U12 = L11^-1 A12 -> A22 -= L21 U12 ->
-//     right half -> swap left half.
-//   Row interchanges are applied to every column of A, matching the
-//   reference's full-row rawSwapRows (fromCol = 0, LU.hs:324-325).
-//   Every U12 = L11^-1 A12 (rawTriSolvePanelTrail, LU.hs:364-407) runs as
-//   inv(L11) (one CTA, blocked inversion in shared memory) times a copy of A12
-//   on the DMMA GEMM: the multipliers are bounded by 1 under partial
-//   pivoting, so the explicit inverse of the unit-lower block is well scaled,
-//   and the block solve leaves the latency-bound substitution kernel.
+//   reference's k = 32 update, LU.hs:311-357).  A panel is one cluster launch
+//   (panel_lu); its row interchanges and U12 = L11^-1 A12
+//   (rawTriSolvePanelTrail, LU.hs:364-407) reach the other columns in one
+//   launch each side of the look-ahead (row_block).  Row interchanges are
+//   applied to every column of A, matching the reference's full-row
+//   rawSwapRows (fromCol = 0, LU.hs:324-325).
 // dpotrf — right-looking blocked Cholesky, kNB = 128: diagonal block in SMEM,
 //   L21 = A21 L11^-T (inverse block times the panel, on the tensor cores), then
 //   A22 -= L21 L21^T as a lower-triangle-only GEMM (SYRK tile skip).  Same
@@ -33,111 +28,81 @@ namespace {
 
 constexpr int kNB = 128;
 
-// Scratch of the inverse-based block solves: inv(L11) (kNB x kNB) and the
-// row-interchange plan.
-struct TrsmScratch {
-  double* Linv;
-  int* plan;  // kSwapPlanInts
-};
 
-// B (w x ncols, ldb) <- inv(unit lower L11) B.  Small blocks (inside a panel)
-// in one fused launch; the panel's row block as inv(L11) times B on the
-// tensor cores, written in place: with m = w <= 128 there is one row of
-// output tiles, so each CTA reads exactly the columns of B that it later
-// overwrites, all of them before its epilogue, and no other CTA reads them.
-// With have_inv, s.Linv already holds inv(L11).
+// B (w x ncols, ldb) <- inv(unit lower L11) B (the no-pivot factorisation's
+// row block).  Small blocks in one fused launch; otherwise inv(L11) (Linv,
+// kNB x kNB scratch) times B on the tensor cores, written in place: with
+// m = w <= 128 there is one row of output tiles, so each CTA reads exactly
+// the columns of B that it later overwrites, all of them before its epilogue,
+// and no other CTA reads them.
 int trsm_unit_lower_gemm(Ctx& c, const double* L11, long long lda, int w, double* B, long long ldb, int ncols,
-                         const TrsmScratch& s, cudaStream_t st, bool have_inv = false) {
+                         double* Linv, cudaStream_t st) {
   if (w <= 0 || ncols <= 0) return LM_OK;
-  if (w <= 64 && ncols <= 128 && !have_inv) {
+  if (w <= 64 && ncols <= 128) {
     Prof p(c, kPhaseTrsm, (double)w * w * ncols, 8.0 * ((double)w * w / 2 + 2.0 * w * ncols), st);
     return trsm_lower_small<double>(L11, lda, w, true, B, ldb, ncols, st);
   }
-  if (!have_inv) {
+  {
     Prof p(c, kPhaseTrsm, (double)w * w * w / 3.0, 8.0 * (double)w * w, st);
-    LM_TRY(tri_inv_lower<double>(L11, lda, w, true, s.Linv, kNB, nullptr, st));
+    LM_TRY(tri_inv_lower<double>(L11, lda, w, true, Linv, kNB, nullptr, st));
   }
   GemmDesc d;
   d.m = w; d.n = ncols; d.k = w;
   d.alpha = 1.0; d.beta = 0.0;
-  d.A = s.Linv; d.lda = kNB;
+  d.A = Linv; d.lda = kNB;
   d.B = B; d.ldb = ldb;
   d.C = B; d.ldc = ldb;
   return dgemm(c, d, st);
 }
 
-// gemm_sms caps the SMs of the panel's own GEMMs (0 = no cap), so that a
-// panel factored beside a trailing update fits on the SMs that update leaves.
-int getrf_panel_rec(Ctx& c, double* A, long long lda, int n, int c0, int w, int pc0, int pw, int* ipiv,
-                    const TrsmScratch& s, cudaStream_t st, int gemm_sms = 0) {
-  const int R = n - c0;
-  const int wmax = panel_leaf_max_width_for(c, R);
-  if (wmax <= 0) return LM_ERR_UNSUPPORTED;
-  if (w <= wmax) {
-    // the leaf also swaps the rest of the panel [pc0, pc0 + pw)
-    Prof p(c, kPhasePanel, (double)R * w * w, 16.0 * R * w, st);
-    return panel_leaf<double>(c, A, lda, n, c0, w, pc0, pw, ipiv, st);
-  }
-  // Split so that column offsets stay multiples of 4 (16-byte TMA alignment).
-  int w1 = (w >= 16) ? std::max(8, (w / 2) & ~7) : std::max(4, (w / 2) & ~3);
-  if (w1 >= w) w1 = w - 4;
-  const int w2 = w - w1;
-  LM_TRY(getrf_panel_rec(c, A, lda, n, c0, w1, pc0, pw, ipiv, s, st, gemm_sms));
-  double* A11 = A + (long long)c0 * lda + c0;
-  LM_TRY(trsm_unit_lower_gemm(c, A11, lda, w1, A11 + w1, lda, w2, s, st));
-  GemmDesc d;
-  d.m = R - w1; d.n = w2; d.k = w1;
-  d.alpha = -1.0; d.beta = 1.0;
-  d.A = A11 + (long long)w1 * lda; d.lda = lda;
-  d.B = A11 + w1; d.ldb = lda;
-  d.C = A11 + (long long)w1 * lda + w1; d.ldc = lda;
-  d.max_sms = gemm_sms;
-  LM_TRY(dgemm(c, d, st));
-  return getrf_panel_rec(c, A, lda, n, c0 + w1, w2, pc0, pw, ipiv, s, st, gemm_sms);
-}
-
 }  // namespace
 
-// SMs left to a panel factored beside the trailing update (the widest panel
-// leaf is a cluster of 16 CTAs of one SM each), and the order from which that
-// look-ahead is used.
+// Order from which a panel (or block column) is factored beside the trailing
+// update, and the SMs that the Cholesky update leaves for it.
 constexpr int kLookaheadSms = 16;
-constexpr int kLookaheadMinN = 2048;
+constexpr int kLookaheadMinN = 384;
 
+// The chain from one panel to the next holds only what the next panel needs:
+// the interchanges, block solve and update of its own 128 columns.  With
+// look-ahead it is then factored on the priority stream while the same three
+// operations run on the rest of the matrix, on the SMs that the panel's
+// cluster leaves.  Nothing waits across the two streams inside a kernel; at
+// worst the panel starts when the update ends.
 int dgetrf(Ctx& c, int n, double* A, long long lda, int* ipiv, cudaStream_t st) {
-  TrsmScratch s;
+  int* plan[2];  // row plans of the current panel and of the one factored beside its update
   {
     void* ws = nullptr;
-    LM_TRY(ctx_workspace(c, 1, sizeof(double) * (size_t)kNB * kNB + sizeof(int) * kSwapPlanInts, &ws));
-    s.Linv = static_cast<double*>(ws);
-    s.plan = reinterpret_cast<int*>(s.Linv + (size_t)kNB * kNB);
+    LM_TRY(ctx_workspace(c, 1, 2 * sizeof(int) * kSwapPlanInts, &ws));
+    plan[0] = static_cast<int*>(ws);
+    plan[1] = plan[0] + kSwapPlanInts;
   }
-  // Look-ahead: once the next panel's columns are updated, that panel is
-  // factored on the priority stream while the rest of the trailing update
-  // runs with a grid that leaves kLookaheadSms SMs free.  Its own GEMMs are
-  // capped to fit there.  Nothing waits across the two streams inside a
-  // kernel; at worst the panel starts when the update ends.
   const int nsm = ctx_num_sms(c);
   const bool la = n >= kLookaheadMinN && nsm > 2 * kLookaheadSms && ctx_lookahead(c);
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   if (la) LM_TRY(ctx_aux(c, &aux, &ev_fork, &ev_join));
-  const int panel_sms = kLookaheadSms;
-  const int rest_sms = nsm - kLookaheadSms;
-  LM_TRY(getrf_panel_rec(c, A, lda, n, 0, std::min(kNB, n), 0, std::min(kNB, n), ipiv, s, st));
+  auto panel = [&](int k0, cudaStream_t s) {
+    const int w = std::min(kNB, n - k0);
+    Prof p(c, kPhasePanel, (double)(n - k0) * w * w, 16.0 * (n - k0) * w, s);
+    return panel_lu<double>(c, A, lda, n, k0, w, ipiv, plan[(k0 / kNB) & 1], s);
+  };
+  LM_TRY(panel(0, st));
   for (int k0 = 0; k0 < n; k0 += kNB) {
     const int w = std::min(kNB, n - k0);
-    // panel k is factored: its interchanges on the columns left and right of it
-    {
-      Prof p(c, kPhaseSwap, 0.0, 32.0 * w * (n - w), st);
-      LM_TRY(laswp<double>(A, lda, n, ipiv, k0, k0 + w, 0, k0, k0 + w, n, ctx_status(c), st, s.plan));
-    }
-    if (k0 + w >= n) break;
     const int m = n - k0 - w;
     const int wn = std::min(kNB, m);  // next panel
+    const int* pl = plan[(k0 / kNB) & 1];
+    auto rows = [&](int ca0, int ca1, int cb0, int cb1) {
+      Prof p(c, kPhaseTrsm, (double)w * w * (cb1 - cb0), 8.0 * (4.0 * w * (ca1 - ca0 + cb1 - cb0) + 0.5 * w * w), st);
+      return row_block<double>(A, lda, pl, k0, w, ca0, ca1, cb0, cb1, st);
+    };
+    if (m <= 0) {
+      LM_TRY(rows(0, k0, n, n));
+      break;
+    }
+    const int nx = k0 + w, rx = nx + wn;  // first columns of the next panel and of the rest
+    LM_TRY(rows(0, 0, nx, rx));
     double* A11 = A + (long long)k0 * lda + k0;
-    // with look-ahead, inv(L11) of this panel was formed beside the previous update
-    LM_TRY(trsm_unit_lower_gemm(c, A11, lda, w, A11 + w, lda, m, s, st, la && k0 > 0));
     GemmDesc d;  // A22 -= L21 U12, the next panel's columns first
     d.m = m; d.n = wn; d.k = w;
     d.alpha = -1.0; d.beta = 1.0;
@@ -152,23 +117,16 @@ int dgetrf(Ctx& c, int n, double* A, long long lda, int* ipiv, cudaStream_t st) 
     if (la) {
       LM_CUDA_TRY(cudaEventRecord(ev_fork, st));
       LM_CUDA_TRY(cudaStreamWaitEvent(aux, ev_fork, 0));
-      LM_TRY(getrf_panel_rec(c, A, lda, n, k0 + w, wn, k0 + w, wn, ipiv, s, aux, panel_sms));
-      if (k0 + w + wn < n) {
-        // the next step's block solve needs inv(L11) of this panel; the
-        // current step's product with the old inverse has already run
-        Prof p(c, kPhaseTrsm, (double)wn * wn * wn / 3.0, 8.0 * (double)wn * wn, aux);
-        LM_TRY(tri_inv_lower<double>(A + (long long)(k0 + w) * lda + k0 + w, lda, wn, true, s.Linv, kNB, nullptr, aux));
-      }
+      LM_TRY(panel(nx, aux));
       LM_CUDA_TRY(cudaEventRecord(ev_join, aux));
-      if (r.n > 0) {
-        r.max_sms = rest_sms;
-        LM_TRY(dgemm(c, r, st));
-      }
-      LM_CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
-    } else {
-      if (r.n > 0) LM_TRY(dgemm(c, r, st));
-      LM_TRY(getrf_panel_rec(c, A, lda, n, k0 + w, wn, k0 + w, wn, ipiv, s, st));
+      r.max_sms = nsm - panel_ctas<double>(c, m);
     }
+    LM_TRY(rows(0, k0, rx, n));
+    if (r.n > 0) LM_TRY(dgemm(c, r, st));
+    if (la)
+      LM_CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
+    else
+      LM_TRY(panel(nx, st));
   }
   return LM_OK;
 }
@@ -274,14 +232,11 @@ int dpotrf(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
 int dgetrf_nopiv(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
   void* ws = nullptr;
   const size_t blk = (size_t)kNB * kNB;
-  LM_TRY(ctx_workspace(c, 1, sizeof(double) * (3 * blk + (size_t)n * kNB) + sizeof(int) * kSwapPlanInts, &ws));
+  LM_TRY(ctx_workspace(c, 1, sizeof(double) * (3 * blk + (size_t)n * kNB), &ws));
   double* Linv = static_cast<double*>(ws);
   double* Ut = Linv + blk;
   double* Uinv = Ut + blk;
   double* W21 = Uinv + blk;
-  TrsmScratch s;
-  s.Linv = Linv;
-  s.plan = reinterpret_cast<int*>(W21 + (size_t)n * kNB);
   for (int j0 = 0; j0 < n; j0 += kNB) {
     const int w = std::min(kNB, n - j0);
     const int R = n - j0 - w;
@@ -293,7 +248,7 @@ int dgetrf_nopiv(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
     if (R <= 0) break;
     double* A12 = A11 + w;
     double* A21 = A11 + (long long)w * lda;
-    LM_TRY(trsm_unit_lower_gemm(c, A11, lda, w, A12, lda, R, s, st));
+    LM_TRY(trsm_unit_lower_gemm(c, A11, lda, w, A12, lda, R, Linv, st));
     {
       Prof p(c, kPhaseTrsm, (double)w * w * w / 3.0, 24.0 * (double)w * w, st);
       LM_TRY(transpose_block(Ut, kNB, A11, lda, w, st));

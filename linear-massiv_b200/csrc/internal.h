@@ -99,12 +99,22 @@ int dgemm(Ctx& c, const GemmDesc& d, cudaStream_t st);
 // Apply row interchanges ipiv[k0..k1) in order (row s <-> row ipiv[s]) to the
 // columns [ca0, ca1) and [cb0, cb1) of A (nrows rows).  A pivot row outside
 // [0, nrows) is skipped and recorded as LM_DEVERR_BOUNDS in status[0].
-// `plan` (kSwapPlanInts ints of device scratch, or null) lets wide updates
-// compose the interchanges once instead of in every column block.
-constexpr int kSwapPlanInts = 1 + 2 * 256 + 15;
 template <typename T>
 int laswp(T* A, long long lda, int nrows, const int* ipiv, int k0, int k1, int ca0, int ca1, int cb0, int cb1,
-          int* status, cudaStream_t st, int* plan = nullptr);
+          int* status, cudaStream_t st);
+
+// Row plan of one panel's interchanges: [0] the number of rows that change
+// place (at most kSwapPlanRows), then their destination rows, then (from
+// 1 + kSwapPlanRows) the rows they come from.
+constexpr int kSwapPlanRows = 256;
+constexpr int kSwapPlanInts = 1 + 2 * kSwapPlanRows + 15;
+// The rest of a panel step on the other columns (row_block.cu): the rows of
+// `plan` moved on columns [ca0, ca1) and [cb0, cb1), and on [cb0, cb1) the
+// block solve  A[k0 : k0 + w, cb0 : cb1) <- inv(L11) A[...]  with the unit
+// lower triangle of the panel's diagonal block (already in its final order).
+template <typename T>
+int row_block(T* A, long long lda, const int* plan, int k0, int w, int ca0, int ca1, int cb0, int cb1,
+              cudaStream_t st);
 
 // All interchanges ipiv[0..n) on a narrow n x nrhs block B at once (one
 // parallel gather into W, n x nrhs scratch, then copied back).
@@ -187,14 +197,17 @@ int dpotrf(Ctx& c, int n, double* A, long long lda, cudaStream_t st);
 int dpotrs(Ctx& c, int n, int nrhs, const double* G, long long lda, double* B, long long ldb,
            cudaStream_t st);
 
-// Panel factorisation kernels (panel.cu): LU of rows [c0, n) x columns
-// [c0, c0 + w) in place, w <= 32, recording ipiv[c0 .. c0 + w) (global rows)
-// and the first zero pivot in status[1].  The leaf's row interchanges are
-// also applied to the other columns of the enclosing panel [pc0, pc0 + pw)
-// (pw <= 128); columns outside it are left to the caller.
+// Panel LU with partial pivoting (panel.cu): rows [c0, n) x columns
+// [c0, c0 + pw) of A in place (pw <= 128; A and its rows 16-byte aligned),
+// recording ipiv[c0 .. c0 + pw) (global rows) and the first zero pivot in
+// status[1].  The panel's own columns are left in their final row order;
+// `plan` (kSwapPlanInts ints of device scratch) receives the rows that
+// changed place, for the other columns (row_block).
 template <typename T>
-int panel_leaf(Ctx& c, T* A, long long lda, int n, int c0, int w, int pc0, int pw, int* ipiv, cudaStream_t st);
-int panel_leaf_max_width_for(Ctx& c, int rows);  // widest leaf one cluster holds for `rows`
+int panel_lu(Ctx& c, T* A, long long lda, int n, int c0, int pw, int* ipiv, int* plan, cudaStream_t st);
+// CTAs (one SM each) that the panel kernel occupies for `rows` rows.
+template <typename T>
+int panel_ctas(Ctx& c, int rows);
 
 // Cholesky of a w x w diagonal block (w <= 128) in place, lower triangle;
 // records the first non-positive pivot (global index base + j + 1) in status[1].

@@ -203,34 +203,12 @@ __global__ void colmax_abs_kernel(const double* V, long long ldv, int rows, int 
 int grid_of(long long total) { return (int)std::max<long long>(1, std::min<long long>(cdivll(total, 256), 2048)); }
 
 // Scratch for the split operands of the 3xTF32 update: L21 -> Ahi/Alo
-// (m x k), U12^T -> Bhi/Blo (n x k); all with leading dimension 128 (k <= 128);
-// Lhi/Llo hold split(inv(L11)) for the block solves (128 x 128).
+// (m x k), U12^T -> Bhi/Blo (n x k); all with leading dimension 128 (k <= 128).
 struct SScratch {
-  float *Ahi, *Alo, *Bhi, *Blo, *Lhi, *Llo;
+  float *Ahi, *Alo, *Bhi, *Blo;
   long long ld;
-  int* plan;  // row-interchange plan (kSwapPlanInts)
+  int* plan[2];  // row plans of the current panel and of the next (kSwapPlanInts)
 };
-
-// B (w x ncols, ldb) <- inv(unit lower L11) B: small blocks (inside a panel)
-// in one fused FP32 launch; otherwise the inverse of the diagonal block (one
-// CTA) times B on the tensor cores as 3xTF32.
-int s_trsm_unit_lower(Ctx& c, const float* L11, long long lda, int w, float* B, long long ldb, int ncols,
-                      SScratch& s, cudaStream_t st, int max_ctas = 0) {
-  if (w <= 0 || ncols <= 0) return LM_OK;
-  if (w <= 64 && ncols <= 128) {
-    Prof p(c, kPhaseTrsm, (double)w * w * ncols, 4.0 * ((double)w * w / 2 + 2.0 * w * ncols), st);
-    return trsm_lower_small<float>(L11, lda, w, true, B, ldb, ncols, st);
-  }
-  {
-    Prof p(c, kPhaseTrsm, (double)w * w * w / 3.0, 12.0 * (double)w * w, st);
-    LM_TRY(tri_inv_lower<float>(L11, lda, w, true, s.Lhi, kNB, s.Llo, st));
-  }
-  dim3 tb(32, 8), tg(cdiv(ncols, 32), cdiv(w, 32));
-  transpose_split_kernel<<<tg, tb, 0, st>>>(s.Bhi, s.Blo, s.ld, B, ldb, w, ncols);
-  count_launch(1);
-  LM_CUDA_TRY(cudaGetLastError());
-  return sgemm_tf32(c, w, ncols, w, 1.0f, s.Lhi, kNB, s.Bhi, s.ld, 0.0f, B, ldb, st, s.Llo, s.Blo, max_ctas);
-}
 
 int s_update(Ctx& c, int m, int n, int k, float* A21, long long lda, const float* U12, float* C, SScratch& s,
              cudaStream_t st, int max_ctas = 0, int prec = LM_IR_PREC_TF32X3) {
@@ -260,104 +238,82 @@ int s_update(Ctx& c, int m, int n, int k, float* A21, long long lda, const float
   return sgemm_tf32(c, m, n, k, -1.0f, s.Ahi, s.ld, s.Bhi, s.ld, 1.0f, C, lda, st, s.Alo, s.Blo, max_ctas);
 }
 
-// max_ctas caps the grids of the panel's own GEMMs (0 = no cap), so that a
-// panel factored beside a trailing update fits on the SMs that update leaves.
-int sgetrf_panel_rec(Ctx& c, float* A, long long lda, int n, int c0, int w, int pc0, int pw, int* ipiv, SScratch& s,
-                     cudaStream_t st, int max_ctas = 0) {
-  const int R = n - c0;
-  const int wmax = panel_leaf_max_width_for(c, R);
-  if (wmax <= 0) return LM_ERR_UNSUPPORTED;
-  if (w <= wmax) {
-    Prof p(c, kPhasePanel, (double)R * w * w, 8.0 * R * w, st);
-    return panel_leaf<float>(c, A, lda, n, c0, w, pc0, pw, ipiv, st);
-  }
-  int w1 = (w >= 16) ? std::max(8, (w / 2) & ~7) : std::max(4, (w / 2) & ~3);
-  if (w1 >= w) w1 = w - 4;
-  const int w2 = w - w1;
-  LM_TRY(sgetrf_panel_rec(c, A, lda, n, c0, w1, pc0, pw, ipiv, s, st, max_ctas));
-  float* A11 = A + (long long)c0 * lda + c0;
-  LM_TRY(s_trsm_unit_lower(c, A11, lda, w1, A11 + w1, lda, w2, s, st, max_ctas));
-  LM_TRY(s_update(c, R - w1, w2, w1, A11 + (long long)w1 * lda, lda, A11 + w1, A11 + (long long)w1 * lda + w1, s, st,
-                  max_ctas));
-  return sgetrf_panel_rec(c, A, lda, n, c0 + w1, w2, pc0, pw, ipiv, s, st, max_ctas);
-}
-
-// Split-operand scratch set carved from `p` (4 n x 128 + 2 128 x 128 floats,
-// then the interchange plan); returns the end of the set.
-char* carve_scratch(SScratch& s, char* p, int n) {
+// Split-operand scratch carved from `p` (4 n x 128 floats, then two row plans).
+void carve_scratch(SScratch& s, char* p, int n) {
   s.ld = kNB;
   s.Ahi = reinterpret_cast<float*>(p);
   s.Alo = s.Ahi + (size_t)n * kNB;
   s.Bhi = s.Alo + (size_t)n * kNB;
   s.Blo = s.Bhi + (size_t)n * kNB;
-  s.Lhi = s.Blo + (size_t)n * kNB;
-  s.Llo = s.Lhi + (size_t)kNB * kNB;
-  s.plan = reinterpret_cast<int*>(s.Llo + (size_t)kNB * kNB);
-  return reinterpret_cast<char*>(s.plan) + ((sizeof(int) * kSwapPlanInts + 255) / 256) * 256;
+  s.plan[0] = reinterpret_cast<int*>(s.Blo + (size_t)n * kNB);
+  s.plan[1] = s.plan[0] + kSwapPlanInts;
 }
 
-size_t scratch_set_bytes(int n) {
-  return sizeof(float) * (4 * (size_t)n * kNB + 2 * (size_t)kNB * kNB) + ((sizeof(int) * kSwapPlanInts + 255) / 256) * 256;
-}
+size_t scratch_bytes(int n) { return sizeof(float) * 4 * (size_t)n * kNB + 2 * sizeof(int) * kSwapPlanInts; }
 
-// SMs left to a panel factored beside the trailing update (the widest panel
-// leaf is a cluster of 16 CTAs of one SM each), and the order from which that
-// look-ahead is used.
+// Order from which the next panel is factored beside the trailing update.
 constexpr int kSLookaheadSms = 16;
-constexpr int kSLookaheadMinN = 2048;
+constexpr int kSLookaheadMinN = 384;
 
 }  // namespace
 
-// FP32 LU with partial pivoting (the same pivot rule as the FP64 path), 128-
-// column panels factored by cluster leaves, U12 = inv(L11) A12 and the
-// updates inside a panel as 3xTF32 on tcgen05; the trailing Schur-complement
-// update, where the flops are, at `prec` (3xTF32, TF32 or BF16).  Look-ahead as in dgetrf:
-// once the next panel's columns are updated, that panel is factored on the
-// priority stream (its own GEMMs capped to the SMs left free) while the rest
-// of the trailing update runs; its interchanges reach the columns right of it
-// after the join.  The two streams use separate split-operand scratch.
+// FP32 LU with partial pivoting (the same pivot rule as the FP64 path): 128-
+// column panels in one cluster launch each, interchanges and U12 = inv(L11)
+// A12 by FP32 substitution (row_block); the trailing Schur-complement update,
+// where the flops are, at `prec` (3xTF32, TF32 or BF16).  Look-ahead as in
+// dgetrf: once the next panel's columns are updated, that panel is factored
+// on the priority stream while the rest of the step runs on the SMs that its
+// cluster leaves.
 int sgetrf(Ctx& c, int n, float* A, long long lda, int* ipiv, cudaStream_t st, int prec) {
   const int nsm = ctx_num_sms(c);
   const bool la = n >= kSLookaheadMinN && nsm > 2 * kSLookaheadSms && ctx_lookahead(c);
   void* ws = nullptr;
-  LM_TRY(ctx_workspace(c, 1, (la ? 2 : 1) * scratch_set_bytes(n), &ws));
-  SScratch s, sa;
-  char* p = carve_scratch(s, static_cast<char*>(ws), n);
-  if (la) carve_scratch(sa, p, n);
+  LM_TRY(ctx_workspace(c, 1, scratch_bytes(n), &ws));
+  SScratch s;
+  carve_scratch(s, static_cast<char*>(ws), n);
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   if (la) LM_TRY(ctx_aux(c, &aux, &ev_fork, &ev_join));
-  LM_TRY(sgetrf_panel_rec(c, A, lda, n, 0, std::min(kNB, n), 0, std::min(kNB, n), ipiv, s, st));
+  auto panel = [&](int k0, cudaStream_t ps) {
+    const int w = std::min(kNB, n - k0);
+    Prof p(c, kPhasePanel, (double)(n - k0) * w * w, 8.0 * (n - k0) * w, ps);
+    return panel_lu<float>(c, A, lda, n, k0, w, ipiv, s.plan[(k0 / kNB) & 1], ps);
+  };
+  LM_TRY(panel(0, st));
   for (int k0 = 0; k0 < n; k0 += kNB) {
     const int w = std::min(kNB, n - k0);
-    {
-      Prof p2(c, kPhaseSwap, 0.0, 16.0 * w * (n - w), st);
-      LM_TRY(laswp<float>(A, lda, n, ipiv, k0, k0 + w, 0, k0, k0 + w, n, ctx_status(c), st, s.plan));
-    }
-    if (k0 + w >= n) break;
     const int m = n - k0 - w;
     const int wn = std::min(kNB, m);  // next panel
+    const int* pl = s.plan[(k0 / kNB) & 1];
+    auto rows = [&](int ca0, int ca1, int cb0, int cb1) {
+      Prof p(c, kPhaseTrsm, (double)w * w * (cb1 - cb0), 4.0 * (4.0 * w * (ca1 - ca0 + cb1 - cb0) + 0.5 * w * w), st);
+      return row_block<float>(A, lda, pl, k0, w, ca0, ca1, cb0, cb1, st);
+    };
+    if (m <= 0) {
+      LM_TRY(rows(0, k0, n, n));
+      break;
+    }
+    const int nx = k0 + w, rx = nx + wn;  // first columns of the next panel and of the rest
+    LM_TRY(rows(0, 0, nx, rx));
     float* A11 = A + (long long)k0 * lda + k0;
-    LM_TRY(s_trsm_unit_lower(c, A11, lda, w, A11 + w, lda, m, s, st));
+    float* A21 = A11 + (long long)w * lda;
     // A22 -= L21 U12 (at the factorisation's precision): the next panel's columns first
-    LM_TRY(s_update(c, m, wn, w, A11 + (long long)w * lda, lda, A11 + w, A11 + (long long)w * lda + w, s, st, 0,
-                    prec));
+    LM_TRY(s_update(c, m, wn, w, A21, lda, A11 + w, A21 + w, s, st, 0, prec));
     const int rest = m - wn;
     if (la) {
       LM_CUDA_TRY(cudaEventRecord(ev_fork, st));
       LM_CUDA_TRY(cudaStreamWaitEvent(aux, ev_fork, 0));
-      LM_TRY(sgetrf_panel_rec(c, A, lda, n, k0 + w, wn, k0 + w, wn, ipiv, sa, aux, kSLookaheadSms));
+      LM_TRY(panel(nx, aux));
       LM_CUDA_TRY(cudaEventRecord(ev_join, aux));
-      if (rest > 0)
-        LM_TRY(s_update(c, m, rest, w, A11 + (long long)w * lda, lda, A11 + w + wn, A11 + (long long)w * lda + w + wn,
-                        s, st, nsm - kSLookaheadSms, prec));
-      LM_CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
-    } else {
-      if (rest > 0)
-        LM_TRY(s_update(c, m, rest, w, A11 + (long long)w * lda, lda, A11 + w + wn, A11 + (long long)w * lda + w + wn,
-                        s, st, 0, prec));
-      LM_TRY(sgetrf_panel_rec(c, A, lda, n, k0 + w, wn, k0 + w, wn, ipiv, s, st));
     }
+    LM_TRY(rows(0, k0, rx, n));
+    if (rest > 0)
+      LM_TRY(s_update(c, m, rest, w, A21, lda, A11 + w + wn, A21 + w + wn, s, st,
+                      la ? nsm - panel_ctas<float>(c, m) : 0, prec));
+    if (la)
+      LM_CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
+    else
+      LM_TRY(panel(nx, st));
   }
   return LM_OK;
 }

@@ -1,31 +1,40 @@
 // Panel kernels: the latency-bound, column-by-column parts of LU and Cholesky.
 //
-// panel_leaf  — partial-pivoting LU of a tall panel (rows [c0, n), up to 32
-//   columns), the B200 replacement for the per-column loop of panelLUFactor
-//   (LU.hs:320-327): rawPivotSearch (K.hs:1541-1556), rawSwapRows
-//   (K.hs:1507-1537) and rawLUEliminateColumnTo (K.hs:1464-1503).
-//   The panel is held in the shared memory of a thread-block cluster (up to 16
-//   CTAs, each owning a contiguous slab of rows, column-major in SMEM).  Per
-//   column: each CTA reduces its slab's |a_ij| with warp shuffles, publishes
-//   (value, row, candidate row, row j) in a double-buffered mailbox, one
-//   cluster barrier, then every CTA reads all mailboxes over distributed shared
-//   memory, picks the pivot (largest |a|, lowest row on ties — the reference's
-//   strict '>' scan), swaps and eliminates its own rows, fusing the next
-//   column's local argmax into the elimination pass.
-//   Each thread keeps its rows in registers in a rotating layout (slot 0 is
-//   always the current column; finished columns move to the end), so that
-//   every column step runs the same compact code: a loop body specialised per
-//   column index does not fit the instruction cache and made each step
-//   fetch-bound.  Rows never move between threads: each carries its logical
-//   row index, an interchange swaps two labels, and the write-back puts every
-//   row at its final position.  So only the candidates travel per column; the
-//   NaN rule for a_jj rides on the candidate of the CTA holding row j.
+// panel_lu  — partial-pivoting LU of a whole panel (rows [c0, n), up to 128
+//   columns) in one launch, the B200 replacement for panelLUFactor's column
+//   loop (LU.hs:320-327: rawPivotSearch K.hs:1541-1556, rawSwapRows
+//   K.hs:1507-1537, rawLUEliminateColumnTo K.hs:1464-1503) together with the
+//   block solves and updates inside the panel.  One thread-block cluster (up
+//   to 16 CTAs); CTA q owns the rows [q rpc, (q + 1) rpc) of the panel from
+//   the first column to the last.  Rows never move while the panel is
+//   factored: each carries its logical index, an interchange swaps two
+//   labels, and the panel's rows are put in order once at the end.  So the
+//   32-column leaves inside a panel need no row exchange of their own:
+//     leaf    : W columns in registers, one thread per row (RPT rows for tall
+//               panels), in micro-panels of MW <= 8 columns;
+//     solve   : the leaf's pivot rows of the remaining columns become U12 =
+//               L11^-1 A12 in shared memory, in every CTA (L11 came with the
+//               pivot rows, so only A12 is read);
+//     update  : every CTA subtracts L21 U12 from its own rows (DMMA for FP64,
+//               FFMA for FP32); the next leaf's columns stay on chip.
+//   The column step is a latency chain: warp vote, CTA barrier, vote over the
+//   warps, one message to every CTA, vote over the CTAs, multipliers, update
+//   of the micro-panel.  Only the micro-panel's 8 columns are on it: they
+//   (with the reciprocal of the leading entry, formed while the warp votes)
+//   are all that a candidate sends, and the rest of the leaf's columns is
+//   updated once per micro-panel with the 8 pivot rows, which their owners
+//   send on the side.  What bounds a column is instruction latency: about 250
+//   instructions at 6 to 7 cycles with one to four warps per scheduler.
+//   A 128-column panel takes 205 us at 500 to 2000 rows (FP64); the 32-column
+//   leaves before it took 63 us each, with 100 us of small solves, products
+//   and interchanges between the four of them (8192 rows).
 //   NaN rule of the reference scan: if |a_jj| is NaN it stays the pivot; NaNs
 //   below it never win.
 //
 // potrf_block — Cholesky of one <=128 x 128 diagonal block in shared memory,
 //   by 32-column panels (rawCholColumnSIMDFrom, K.hs:2137-2195, for a
 //   diagonal panel).
+#include <algorithm>
 #include <climits>
 
 #include "common.cuh"
@@ -37,446 +46,817 @@ void count_launch(int n);
 
 namespace {
 
-constexpr int kLeafThreads = 512;
-constexpr int kLeafRowsTimesW = 16384;  // rows per CTA * leaf width (128 KB of FP64)
-static_assert(kLeafThreads / 32 >= 16, "one pushing warp per CTA of the largest (16-CTA) cluster");
-
-template <typename T>
-__device__ __forceinline__ T absval(T x) {
-  T a = x < T(0) ? -x : x;
-  return (a != a) ? T(-1) : a;  // NaN never wins the scan
-}
+constexpr int kPanelNB = 128;      // widest panel
+constexpr int kPanelThreads = 512; // most threads per CTA (one row of the leaf each, times RPT)
+constexpr int kPanelCtas = 16;     // largest cluster
 
 // The pivot order of the reference's scan (strict '>' from row j down): the
-// larger |a| wins, the lower row on ties, NaN never wins.  Scan values
-// (absval's: -1 or >= 0) become integers in that order: 0 for -1, 1 for zero
-// (either sign), the IEEE bits + 1 above, which grow with the value.  A warp then reduces (key, row) with three redux.sync
-// instead of five shuffle rounds of (value, row) pairs.
+// larger |a| wins, the lower row on ties, NaN never wins.  |a| becomes an
+// integer key in that order, its IEEE bits, so that a warp reduces it with
+// redux.sync.  NaN gets the key of zero: row j, which has the lowest label, is
+// always among the candidates, so neither ever beats it.  Row j with a NaN
+// a_jj stays the pivot (the reference scan starts at row j and NaN never
+// compares greater): kForced beats every other key.
 template <typename T>
-__device__ __forceinline__ unsigned long long scan_key(T v) {
-  if (!(v >= T(0))) return 0ull;
-  if (v == T(0)) return 1ull;
-  if constexpr (sizeof(T) == 8)
-    return (unsigned long long)__double_as_longlong((double)v) + 1ull;
-  else
-    return (unsigned long long)__float_as_uint((float)v) + 1ull;
-}
-// Row j with a NaN a_jj stays the pivot (the reference scan starts at row j
-// and NaN never compares greater): its key beats every other.
-constexpr unsigned long long kForcedKey = ~0ull;
-// A key in the message's T-sized slot, bit for bit (float keys fit 32 bits).
-template <typename T>
-__device__ __forceinline__ T key_to_msg(unsigned long long k) {
-  if constexpr (sizeof(T) == 8)
-    return (T)__longlong_as_double((long long)k);
-  else
-    return (T)__uint_as_float(k == kForcedKey ? 0xffffffffu : (unsigned)k);
-}
-template <typename T>
-__device__ __forceinline__ unsigned long long msg_to_key(T m) {
-  if constexpr (sizeof(T) == 8) {
-    return (unsigned long long)__double_as_longlong((double)m);
-  } else {
-    const unsigned b = __float_as_uint((float)m);
-    return b == 0xffffffffu ? kForcedKey : (unsigned long long)b;
+struct PivKey;
+template <>
+struct PivKey<double> {
+  using K = unsigned long long;
+  static constexpr K kForced = ~0ull;
+  __device__ static K of(double x) {
+    const K u = (K)__double_as_longlong(x) & 0x7fffffffffffffffull;
+    return u > 0x7ff0000000000000ull ? 0ull : u;
   }
+  // the reciprocal of a pivot in this range and the remainders formed with
+  // it neither overflow nor lose bits to underflow
+  __device__ static bool safe(double p) { const double a = fabs(p); return a > 0x1p-500 && a < 0x1p500; }
+  // 1 / p to about an ulp: the hardware estimate and two Newton steps
+  __device__ static double rcp(double p) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(p));
+    r = fma(r, fma(-p, r, 1.0), r);
+    return fma(r, fma(-p, r, 1.0), r);
+  }
+};
+template <>
+struct PivKey<float> {
+  using K = unsigned;
+  static constexpr K kForced = ~0u;
+  __device__ static K of(float x) {
+    const K u = __float_as_uint(x) & 0x7fffffffu;
+    return u > 0x7f800000u ? 0u : u;
+  }
+  __device__ static bool safe(float p) { const float a = fabsf(p); return a > 0x1p-60f && a < 0x1p60f; }
+  __device__ static float rcp(float p) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(p));
+    return fmaf(r, fmaf(-p, r, 1.f), r);
+  }
+};
+
+// Lane (the same in every lane) holding the warp's best (key, label): the
+// largest key, then the lowest label.  Lanes without a candidate pass key 0
+// and label INT_MAX.  Usually one redux.sync and one vote: the later rounds
+// run only when several lanes share the leading bits.
+__device__ __forceinline__ int warp_winner(unsigned key, int label) {
+  __syncwarp();  // reconverge: a split warp would serialise every *_sync below
+  unsigned b = __ballot_sync(0xffffffffu, key == __reduce_max_sync(0xffffffffu, key));
+  if (b & (b - 1)) {
+    const unsigned l = (b >> (threadIdx.x & 31)) & 1 ? (unsigned)label : 0xffffffffu;
+    b = __ballot_sync(0xffffffffu, l == __reduce_min_sync(0xffffffffu, l));
+  }
+  return __ffs(b) - 1;
 }
-// Every lane receives the warp's best (key, row) in the pivot order: the
-// largest key, then the lowest row (rows are >= 0, or INT_MAX for none).
-__device__ __forceinline__ void warp_best(unsigned long long& key, int& row) {
-  // reconverge first: after the data-dependent branches and bounded spins of
-  // a column step a warp can arrive split, and every *_sync below would then
-  // serialise its halves
+__device__ __forceinline__ int warp_winner(unsigned long long key, int label) {
   __syncwarp();
-  const unsigned khi = (unsigned)(key >> 32), klo = (unsigned)key;
-  const unsigned hi = __reduce_max_sync(0xffffffffu, khi);
-  const unsigned lo = __reduce_max_sync(0xffffffffu, khi == hi ? klo : 0u);
-  const unsigned long long best = ((unsigned long long)hi << 32) | lo;
-  row = (int)__reduce_min_sync(0xffffffffu, key == best ? (unsigned)row : 0xffffffffu);
-  key = best;
+  const unsigned hi = (unsigned)(key >> 32);
+  unsigned b = __ballot_sync(0xffffffffu, hi == __reduce_max_sync(0xffffffffu, hi));
+  if (b & (b - 1)) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lo = (b >> lane) & 1 ? (unsigned)key : 0u;
+    b &= __ballot_sync(0xffffffffu, lo == __reduce_max_sync(0xffffffffu, lo));
+    if (b & (b - 1)) {
+      const unsigned l = (b >> lane) & 1 ? (unsigned)label : 0xffffffffu;
+      b &= __ballot_sync(0xffffffffu, l == __reduce_min_sync(0xffffffffu, l));
+    }
+  }
+  return __ffs(b) - 1;
 }
 
-// Per-column message pushed into every CTA of the cluster (T elements), one
-// per source CTA: [0] the scan key of its best candidate (bit pattern, see
-// scan_key; kForcedKey when that row is row j with a NaN a_jj), [1] that
-// row's logical index relative to c0 (or -1), [2..3] unused, [4, 4 + W) the
-// row in the rotated register layout.
-template <typename T, int W>
+// The candidate that each CTA sends to every CTA of the cluster, once per
+// column: 16-byte chunks, header then the micro-panel's part of the row in
+// the rotated register layout.
+template <typename T, int MW>
 struct LeafMsg {
-  static constexpr int N = 4 + W;
-  static constexpr int BYTES = N * (int)sizeof(T);
-  static constexpr int CHUNKS = BYTES / 16;
-  static constexpr int PER_CHUNK = 16 / (int)sizeof(T);
-  static_assert(BYTES % 16 == 0, "message must be a whole number of 16-byte chunks");
+  typename PivKey<T>::K key;  // PivKey of the candidate (kForced: row j with a NaN a_jj)
+  int label;                  // its logical row in the panel, or INT_MAX: no candidate
+  int row;                    // its row in the sending CTA
+  T rcp;                      // reciprocal of its leading entry
+  alignas(16) T v[MW];
 };
 
-template <typename T, int W>
-struct LeafSmem {
-  using M = LeafMsg<T, W>;
-  static constexpr size_t cand_off = 0;                                    // T[2][16][N]
-  static constexpr size_t outc_off = cand_off + 2 * 16 * (size_t)M::BYTES;  // T[N] outgoing candidate
-  static constexpr size_t bar_off = outc_off + (size_t)M::BYTES;            // uint64_t[2]
-  static constexpr size_t wkey_off = bar_off + 16;                          // uint64_t[16] warp best keys
-  static constexpr size_t widx_off = wkey_off + 16 * sizeof(unsigned long long);  // int[16] their rows
-  static constexpr size_t hist_off = widx_off + 16 * sizeof(int);           // int[W] pivot rows
-  static constexpr size_t trow_off = hist_off + W * sizeof(int);            // int[2W] touched rows
-  static constexpr size_t tsrc_off = trow_off + 2 * W * sizeof(int);        // int[2W] their sources
-  static constexpr size_t tm_off = tsrc_off + 2 * W * sizeof(int);          // int touched count
-  static constexpr size_t stage_off = (tm_off + sizeof(int) + 15) / 16 * 16;
-  // One region, used twice: first the CTA's slab (rpc rows x W, row stride
-  // W + 1) for coalesced loads and write-back, followed by the rows' final
-  // logical indices (rpc ints), then the swap staging for the other panel
-  // columns (2W rows x up to 128 columns, split over the cluster).
-  static constexpr int SLD = W + 1;
-  static size_t stage_elems(int C) { return (size_t)(2 * W * 128 + C - 1) / C; }
-  __host__ __device__ static size_t slab_elems(int rpc) { return (size_t)rpc * SLD; }
-  static size_t region_elems(int rpc, int C) {
-    const size_t slab = slab_elems(rpc) + ((size_t)rpc * sizeof(int) + sizeof(T) - 1) / sizeof(T);
-    return slab > stage_elems(C) ? slab : stage_elems(C);
+template <typename T, int W_, int RPT>
+struct PanelCfg {
+  static constexpr int W = W_;
+  static constexpr int MW = W < 8 ? W : 8;  // micro-panel width
+  static constexpr int ZW = W - MW;         // the leaf's columns outside the micro-panel
+  using Msg = LeafMsg<T, MW>;
+  static constexpr int MSG_CHUNKS = (int)sizeof(Msg) / 16;
+  static_assert(sizeof(Msg) % 16 == 0 && MSG_CHUNKS <= 32, "whole 16-byte chunks, one per lane");
+  static constexpr int SLD = W + 16 / (int)sizeof(T);  // slab row stride: 16-byte rows, distinct banks
+  // U12 row stride; = 4 (mod 16) keeps the DMMA operand reads conflict-free
+  static constexpr int LDU = kPanelNB - W + (W >= 8 ? 4 : 8);
+  static constexpr size_t cand = 0;                                    // Msg[2][16] received
+  static constexpr size_t wmsg = cand + 2 * kPanelCtas * sizeof(Msg);  // Msg[2][16] one per warp
+  static constexpr size_t bars = wmsg + 2 * 16 * sizeof(Msg);          // uint64_t[3]
+  static constexpr size_t zrow = bars + 32;                            // T[MW][ZW] pivot rows, other columns
+  static constexpr size_t prow = zrow + MW * ZW * sizeof(T);           // int[2][W] pivot rows (panel-relative)
+  static constexpr size_t list = (prow + 2 * W * 4 + 15) / 16 * 16;    // int[2][256] row plan
+  static constexpr size_t l11 = list + 2 * kSwapPlanRows * 4;          // T[W][SLD], L11 by columns
+  static constexpr size_t us = l11 + W * SLD * sizeof(T);              // T[W][LDU]
+  static constexpr size_t lab = us + (size_t)W * LDU * sizeof(T);      // int[rpc]
+  static size_t slab_off(int rpc) { return lab + ((size_t)rpc * 4 + 15) / 16 * 16; }
+  // the slab, which also stages the moved rows 8 columns at a time
+  __host__ __device__ static int slab_elems(int rpc) {
+    return rpc * SLD > kSwapPlanRows * 8 ? rpc * SLD : kSwapPlanRows * 8;
   }
-  static size_t bytes(int rpc, int C) { return stage_off + region_elems(rpc, C) * sizeof(T); }
+  static size_t bytes(int rpc) { return slab_off(rpc) + (size_t)slab_elems(rpc) * sizeof(T); }
 };
 
-template <typename T>
-__device__ __forceinline__ void pack16(const T* src, uint32_t (&w)[4]) {
+// Block of 32 rows x BW columns of the in-panel update: C -= L U with L
+// (rows r0.., W columns) in the slab and U (W x BW) in shared memory.  C comes
+// from global memory; the result goes back there, or for the next leaf's
+// columns (`keep`) into the slab rows.  Rows that are finished (label < done)
+// keep their global contents.
+template <typename T, int W, int SLD, int LDU, int BW>
+__device__ __forceinline__ void panel_update(T* slab, const T* U, const int* lab, int done, int r0, int rcnt, T* C,
+                                             long long lda, int nc, bool keep) {
+  const int lane = threadIdx.x & 31;
   if constexpr (sizeof(T) == 8) {
-    const unsigned long long a = (unsigned long long)__double_as_longlong((double)src[0]);
-    const unsigned long long b = (unsigned long long)__double_as_longlong((double)src[1]);
-    w[0] = (uint32_t)a; w[1] = (uint32_t)(a >> 32); w[2] = (uint32_t)b; w[3] = (uint32_t)(b >> 32);
-  } else {
-    w[0] = __float_as_uint((float)src[0]); w[1] = __float_as_uint((float)src[1]);
-    w[2] = __float_as_uint((float)src[2]); w[3] = __float_as_uint((float)src[3]);
-  }
-}
-
-// Push a message staged in this CTA's shared memory (`msg`) to the same
-// offset `slot` in CTA d of the cluster, completing on its `bar`; one lane
-// per 16-byte chunk.
-template <typename T, int W>
-__device__ __forceinline__ void push_one(const T* msg, T* slot, uint64_t* bar, int d, int lane) {
-  using M = LeafMsg<T, W>;
-  static_assert(M::CHUNKS <= 32, "one chunk per lane");
-  if (lane < M::CHUNKS) {
-    uint32_t w4[4];
-    pack16<T>(msg + lane * M::PER_CHUNK, w4);
-    st_async_16(dsmem_map(slot, d) + lane * 16, dsmem_map(bar, d), w4[0], w4[1], w4[2], w4[3]);
-  }
-}
-
-template <typename T, int W>
-__global__ void __launch_bounds__(kLeafThreads, 1)
-    panel_leaf_kernel(T* A, long long lda, int n, int c0, int w, int rpc, int pc0, int pw, int* ipiv,
-                      int* status) {
-  using L = LeafSmem<T, W>;
-  using M = LeafMsg<T, W>;
-  extern __shared__ __align__(16) unsigned char sm[];
-  T* cand = reinterpret_cast<T*>(sm + L::cand_off);
-  T* outc = reinterpret_cast<T*>(sm + L::outc_off);
-  uint64_t* rbar = reinterpret_cast<uint64_t*>(sm + L::bar_off);
-  unsigned long long* wkey = reinterpret_cast<unsigned long long*>(sm + L::wkey_off);
-  int* widx = reinterpret_cast<int*>(sm + L::widx_off);
-  int* hist = reinterpret_cast<int*>(sm + L::hist_off);
-  int* trow = reinterpret_cast<int*>(sm + L::trow_off);
-  int* tsrc = reinterpret_cast<int*>(sm + L::tsrc_off);
-  int* tm = reinterpret_cast<int*>(sm + L::tm_off);
-  T* stage = reinterpret_cast<T*>(sm + L::stage_off);
-
-  const int q = (int)cluster_ctarank();
-  const int C = (int)cluster_nctarank();
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int R = n - c0;
-  const int rbeg = q * rpc;
-  const int rcnt = max(0, min(rpc, R - rbeg));
-  constexpr int RPT = kLeafRowsTimesW / W / kLeafThreads;  // rows per thread (= 32 / W)
-  static_assert(RPT * W == kLeafRowsTimesW / kLeafThreads, "slab must split evenly");
-
-  if (tid == 0) {
-    mbar_init(&rbar[0], 1);
-    mbar_init(&rbar[1], 1);
-    fence_barrier_init();
-  }
-  // This thread's rows of the slab, in registers: row r = tid + u * threads.
-  // The slab through shared memory: each warp instruction reads 32 / W whole
-  // rows (coalesced), then every thread takes its rows from there.
-  constexpr int SLD = L::SLD;
-  constexpr int RPI = 32 / W;  // rows per warp instruction
-  T* slab = stage;
-  for (int r = warp * RPI + lane / W; r < rcnt; r += (kLeafThreads / 32) * RPI) {
-    const int c = lane % W;
-    slab[r * SLD + c] = c < w ? A[(long long)(c0 + rbeg + r) * lda + c0 + c] : T(0);
-  }
-  __syncthreads();
-  T x[RPT][W];
+    const int gq = lane >> 2, tq = lane & 3;
+    double acc[2][BW / 8][4];
+    bool live[2][2];
 #pragma unroll
-  for (int u = 0; u < RPT; ++u) {
-    const int r = tid + u * kLeafThreads;
+    for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-    for (int c = 0; c < W; ++c) x[u][c] = r < rcnt ? slab[r * SLD + c] : T(0);
-  }
-  cluster_sync_all();  // every CTA's barriers exist before anyone pushes into them
-
-  // logical row (relative to c0) of each of this thread's rows
-  int lr[RPT];
+      for (int h = 0; h < 2; ++h) {
+        const int r = r0 + mi * 16 + h * 8 + gq;
+        live[mi][h] = r < rcnt && lab[r] >= done;
 #pragma unroll
-  for (int u = 0; u < RPT; ++u) lr[u] = rbeg + tid + u * kLeafThreads;
-  // this thread's best candidate for the next column: (key, logical row)
-  unsigned long long bk = 0ull;
-  int bi = INT_MAX;
-#pragma unroll
-  for (int u = 0; u < RPT; ++u) {
-    const int r = tid + u * kLeafThreads;
-    if (r < rcnt) {
-      const unsigned long long k = scan_key(absval(x[u][0]));
-      if (k > bk || (k == bk && lr[u] < bi)) { bk = k; bi = lr[u]; }
-    }
-  }
-
-  bool timed_out = false;
-  // Column j's step.  Register layout of a row at step j: slot c < W - j holds
-  // column j + c, slot W - j + i holds the finished column i.
-#pragma unroll 1
-  for (int j = 0; j < w; ++j) {
-    const int par = j & 1;
-    if (tid == 0) mbar_arrive_expect_tx(&rbar[par], (uint32_t)(C * M::BYTES));
-    // row j with a NaN a_jj is this CTA's candidate whatever else it holds
-#pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      const int r = tid + u * kLeafThreads;
-      if (r < rcnt && lr[u] == j && x[u][0] != x[u][0]) { bk = kForcedKey; bi = j; }
-    }
-    // ---- CTA argmax: warp reduction, one barrier, every warp reduces ----
-    warp_best(bk, bi);
-    if (lane == 0) { wkey[warp] = bk; widx[warp] = bi; }
-    __syncthreads();
-    {
-      const unsigned long long k0 = lane < kLeafThreads / 32 ? wkey[lane] : 0ull;
-      const int i0 = lane < kLeafThreads / 32 ? widx[lane] : INT_MAX;
-      unsigned long long k = k0;
-      int i = i0;
-      warp_best(k, i);
-      // the warp holding the CTA's best row stages and pushes it (warp 0 if none)
-      const int wo = i == INT_MAX ? 0 : __ffs(__ballot_sync(0xffffffffu, k0 == k && i0 == i)) - 1;
-      if (warp == wo) {
-        if (i != INT_MAX) {
-#pragma unroll
-          for (int u = 0; u < RPT; ++u)
-            if (tid + u * kLeafThreads < rcnt && lr[u] == i) {
-#pragma unroll
-              for (int c = 0; c < W; ++c) outc[4 + c] = x[u][c];
-            }
-        } else if (lane < W) {
-          outc[4 + lane] = T(0);
-        }
-        if (lane == 0) {
-          outc[0] = key_to_msg<T>(k);
-          outc[1] = i != INT_MAX ? T(i) : T(-1);
-          outc[2] = T(0);
-          outc[3] = T(0);
+        for (int ni = 0; ni < BW / 8; ++ni) {
+          const int c = ni * 8 + 2 * tq;
+          double2 v = make_double2(0.0, 0.0);
+          if (live[mi][h]) {
+            const double* p = C + (long long)r * lda + c;
+            if (c + 1 < nc) v = *reinterpret_cast<const double2*>(p);
+            else if (c < nc) v.x = *p;
+          }
+          acc[mi][ni][2 * h] = v.x;
+          acc[mi][ni][2 * h + 1] = v.y;
         }
       }
-    }
-    // the staged candidate goes out from C warps at once: warp d sends it to
-    // CTA d, one 16-byte chunk per lane (one warp sending all C copies took
-    // about 900 cycles per column)
-    __syncthreads();
-    if (warp < C) push_one<T, W>(outc, cand + ((size_t)par * 16 + q) * M::N, &rbar[par], warp, lane);
-    // ---- wait for the C candidates ----
-    if (!timed_out && !mbar_wait_spin(&rbar[par], (uint32_t)((j >> 1) & 1), status)) timed_out = true;
-
-    const T* rc = cand + (size_t)par * 16 * M::N;
-    int i = lane < C ? (int)rc[lane * M::N + 1] : INT_MAX;
-    if (i < 0) i = INT_MAX;
-    int qw;
-    {
-      const unsigned long long mine = lane < C ? msg_to_key(rc[lane * M::N + 0]) : 0ull;
-      const int my_row = i;
-      unsigned long long k = mine;
-      warp_best(k, i);
-      qw = __ffs(__ballot_sync(0xffffffffu, mine == k && my_row == i)) - 1;  // the winning CTA
-    }
-    // (row j itself is always a candidate, so some CTA wins; the fallback
-    // only keeps the indexing in bounds)
-    const int p = (i == INT_MAX || qw >= C) ? j : i;
-    const T* prow = rc + ((i == INT_MAX || qw >= C) ? 0 : qw) * M::N + 4;
-    const T piv = prow[0];
-    if (tid == 0) hist[j] = p;
-    if (q == 0 && tid == 0) {
-      ipiv[c0 + j] = c0 + p;
-      if (piv == T(0)) atomicCAS(status + 1, 0, c0 + j + 1);
-    }
-
-    // ---- interchange labels, eliminate own rows in registers, scan column j+1 ----
-    bk = 0ull;
-    bi = INT_MAX;
+    __syncwarp();
+#pragma unroll 2
+    for (int k = 0; k < W; k += 4) {
+      double a[2][2], b[BW / 8];
 #pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      const int r = tid + u * kLeafThreads;
-      if (r < rcnt) {
-        if (lr[u] == p)
-          lr[u] = j;
-        else if (lr[u] == j)
-          lr[u] = p;
-        if (lr[u] > j) {
-          const T mult = x[u][0] / piv;
-          x[u][0] = mult;
+      for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-          for (int c = 1; c < W; ++c)
-            if (c < W - j) x[u][c] = fma(-mult, prow[c], x[u][c]);
-          if (j + 1 < w) {
-            const unsigned long long k1 = scan_key(absval(x[u][1]));
-            if (k1 > bk || (k1 == bk && lr[u] < bi)) { bk = k1; bi = lr[u]; }
+        for (int h = 0; h < 2; ++h) a[mi][h] = -slab[(r0 + mi * 16 + h * 8 + gq) * SLD + k + tq];
+#pragma unroll
+      for (int ni = 0; ni < BW / 8; ++ni) b[ni] = U[(k + tq) * LDU + ni * 8 + gq];
+#pragma unroll
+      for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < BW / 8; ++ni) dmma_16x8x4(acc[mi][ni], a[mi][0], a[mi][1], b[ni]);
+    }
+    if (keep) __syncwarp();  // every lane has read its slab operands
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = r0 + mi * 16 + h * 8 + gq;
+#pragma unroll
+        for (int ni = 0; ni < BW / 8; ++ni) {
+          const int c = ni * 8 + 2 * tq;
+          const double2 v = make_double2(acc[mi][ni][2 * h], acc[mi][ni][2 * h + 1]);
+          if (keep && c < W) {
+            if (r < rcnt) {
+              slab[r * SLD + c] = c < nc ? v.x : 0.0;
+              slab[r * SLD + c + 1] = c + 1 < nc ? v.y : 0.0;
+            }
+          } else if (live[mi][h]) {
+            double* p = C + (long long)r * lda + c;
+            if (c + 1 < nc) *reinterpret_cast<double2*>(p) = v;
+            else if (c < nc) *p = v.x;
           }
         }
       }
-      // column j's final value moves to the end
-      const T t0 = x[u][0];
+  } else {
+    // lane = (row group rg, column group tq): rows r0 + 8 i + rg, columns tq CT ..
+    constexpr int CT = BW / 4;
+    const int rg = lane >> 2, tq = lane & 3;
+    float acc[4][CT];
+    bool live[4];
 #pragma unroll
-      for (int c = 0; c + 1 < W; ++c) x[u][c] = x[u][c + 1];
-      x[u][W - 1] = t0;
-    }
-    // The buffers of this parity are rewritten two columns later; the
-    // barrier at the top of the next column orders these reads before this
-    // CTA pushes again, and no CTA can run two columns ahead of another.
-  }
-  // a leaf narrower than W stops w steps into the rotation: finish it
-#pragma unroll 1
-  for (int k = w; k < W; ++k)
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + 8 * i + rg;
+      live[i] = r < rcnt && lab[r] >= done;
 #pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      const T t0 = x[u][0];
-#pragma unroll
-      for (int c = 0; c + 1 < W; ++c) x[u][c] = x[u][c + 1];
-      x[u][W - 1] = t0;
-    }
-  // Nobody may leave while others can still write into it.
-  cluster_sync_all();
-  // write-back through the slab, coalesced like the load, each row to its
-  // logical position
-  int* lrow = reinterpret_cast<int*>(slab + L::slab_elems(rpc));
-#pragma unroll
-  for (int u = 0; u < RPT; ++u) {
-    const int r = tid + u * kLeafThreads;
-    if (r < rcnt) {
-#pragma unroll
-      for (int c = 0; c < W; ++c) slab[r * SLD + c] = x[u][c];
-      lrow[r] = lr[u];
-    }
-  }
-  __syncthreads();
-  for (int r = warp * RPI + lane / W; r < rcnt; r += (kLeafThreads / 32) * RPI) {
-    const int c = lane % W;
-    if (c < w) A[(long long)(c0 + lrow[r]) * lda + c0 + c] = slab[r * SLD + c];
-  }
-  __syncthreads();  // the region is the swap staging from here on
-  // This leaf's interchanges on the other columns of the enclosing panel
-  // [pc0, pc0 + pw): compose them (rows relative to c0), gather every touched
-  // row's source over the cluster, barrier, scatter.
-  const int ocols = pw - w;
-  if (ocols > 0) {
-    // Touched rows: 0 .. w-1, then each pivot row >= w in order of first
-    // use; the source of row r is tau_0(tau_1(... tau_{w-1}(r))), walking
-    // the interchanges backwards.  One warp (w <= 32).
-    if (warp == 0) {
-      const int pr = lane < w ? hist[lane] : -1;
-      bool fresh = lane < w && pr >= w;
-      for (int jj = 0; jj < lane && jj < w; ++jj)
-        if (hist[jj] == pr) fresh = false;
-      __syncwarp();
-      const unsigned bal = __ballot_sync(0xffffffffu, fresh);
-      if (lane < w) trow[lane] = lane;
-      if (fresh) trow[w + __popc(bal & ((1u << lane) - 1u))] = pr;
-      const int m = w + __popc(bal);
-      __syncwarp();
-      for (int e = lane; e < m; e += 32) {
-        int r = trow[e];
-        for (int jj = w - 1; jj >= 0; --jj) {
-          const int h = hist[jj];
-          if (r == jj) r = h;
-          else if (r == h) r = jj;
-        }
-        tsrc[e] = r;
+      for (int c = 0; c < CT; ++c) {
+        const int cc = tq * CT + c;
+        acc[i][c] = live[i] && cc < nc ? C[(long long)r * lda + cc] : 0.f;
       }
-      if (lane == 0) *tm = m;
     }
-    __syncthreads();
-    const int m = *tm;
-    const long long total = (long long)m * ocols;
-    const long long chunk = (total + C - 1) / C;
-    const long long e0 = q * chunk, e1 = min(total, e0 + chunk);
-    const int left = c0 - pc0;  // other columns: [pc0, c0) then [c0 + w, pc0 + pw)
+    __syncwarp();
 #pragma unroll 4
-    for (long long e = e0 + tid; e < e1; e += kLeafThreads) {
-      const int ii = (int)(e / ocols), oc = (int)(e % ocols);
-      const int col = oc < left ? pc0 + oc : c0 + w + (oc - left);
-      if (tsrc[ii] != trow[ii]) stage[e - e0] = A[(long long)(c0 + tsrc[ii]) * lda + col];
+    for (int k = 0; k < W; ++k) {
+      float a[4], b[CT];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = slab[(r0 + 8 * i + rg) * SLD + k];
+#pragma unroll
+      for (int c = 0; c < CT; ++c) b[c] = U[k * LDU + tq * CT + c];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < CT; ++c) acc[i][c] = fmaf(-a[i], b[c], acc[i][c]);
     }
-    cluster_sync_all();
-    for (long long e = e0 + tid; e < e1; e += kLeafThreads) {
-      const int ii = (int)(e / ocols), oc = (int)(e % ocols);
-      const int col = oc < left ? pc0 + oc : c0 + w + (oc - left);
-      if (tsrc[ii] != trow[ii]) A[(long long)(c0 + trow[ii]) * lda + col] = stage[e - e0];
+    if (keep) __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + 8 * i + rg;
+#pragma unroll
+      for (int c = 0; c < CT; ++c) {
+        const int cc = tq * CT + c;
+        if (keep && cc < W) {
+          if (r < rcnt) slab[r * SLD + cc] = cc < nc ? acc[i][c] : 0.f;
+        } else if (live[i] && cc < nc) {
+          C[(long long)r * lda + cc] = acc[i][c];
+        }
+      }
     }
   }
 }
 
-int g_max_cluster[kMaxDevices] = {};
+// x / p for a pivot p whose correctly rounded reciprocal is r: the quotient
+// estimate x r corrected once by its exact remainder (Markstein 1990).
+template <typename T>
+__device__ __forceinline__ T div_by(T x, T p, T r) {
+  const T q = x * r;
+  return fma(fma(-p, q, x), r, q);
+}
 
-template <typename T, int W>
-int launch_leaf(Ctx& c, T* A, long long lda, int n, int c0, int w, int pc0, int pw, int* ipiv, cudaStream_t st) {
+// N elements between a thread's registers and 16-byte aligned shared memory.
+template <typename T, int N>
+__device__ __forceinline__ void vec_load(T* x, const T* p) {
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll
+    for (int c = 0; c < N; c += 2) {
+      const double2 v = *reinterpret_cast<const double2*>(p + c);
+      x[c] = v.x; x[c + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < N; c += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(p + c);
+      x[c] = v.x; x[c + 1] = v.y; x[c + 2] = v.z; x[c + 3] = v.w;
+    }
+  }
+}
+template <typename T, int N>
+__device__ __forceinline__ void vec_store(T* p, const T* x) {
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll
+    for (int c = 0; c < N; c += 2) *reinterpret_cast<double2*>(p + c) = make_double2(x[c], x[c + 1]);
+  } else {
+#pragma unroll
+    for (int c = 0; c < N; c += 4) *reinterpret_cast<float4*>(p + c) = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
+  }
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// x <- L^-1 x for the unit lower triangle of order N held by columns in
+// shared memory (column k at l + k ld): by columns, so that the updates of
+// one step are independent, with 16-byte loads of L.
+template <typename T, int N>
+__device__ __forceinline__ void unit_lower_solve(T (&x)[N], const T* l, int ld) {
+  constexpr int V = 16 / (int)sizeof(T);
+#pragma unroll
+  for (int k = 0; k + 1 < N; ++k)
+#pragma unroll
+    for (int i = (k + 1) / V * V; i < N; i += V) {
+      T c[V];
+      vec_load<T, V>(c, l + k * ld + i);
+#pragma unroll
+      for (int e = 0; e < V; ++e)
+        if (i + e > k) x[i + e] = fma(-c[e], x[k], x[i + e]);
+    }
+}
+
+// plan: [0] the number of rows of the panel that change place, then their
+// destination rows and (kSwapPlanInts layout) their source rows.
+template <typename T, int W, int RPT>
+__global__ void __launch_bounds__(kPanelThreads, 1)
+    panel_lu_kernel(T* A, long long lda, int n, int c0, int pw, int rpc, unsigned slab_off, int* ipiv, int* plan,
+                    int* status) {
+  using Cfg = PanelCfg<T, W, RPT>;
+  using Msg = typename Cfg::Msg;
+  using Key = typename PivKey<T>::K;
+  constexpr int SLD = Cfg::SLD, LDU = Cfg::LDU, MW = Cfg::MW, ZW = Cfg::ZW;
+  constexpr int V = 16 / (int)sizeof(T);
+  extern __shared__ __align__(16) unsigned char sm[];
+  Msg* cand = reinterpret_cast<Msg*>(sm + Cfg::cand);
+  Msg* wmsg = reinterpret_cast<Msg*>(sm + Cfg::wmsg);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + Cfg::bars);  // candidates (by parity), pivot rows
+  T* zrow = reinterpret_cast<T*>(sm + Cfg::zrow);
+  int* prow_id = reinterpret_cast<int*>(sm + Cfg::prow);  // of this leaf and the one before
+  int* list = reinterpret_cast<int*>(sm + Cfg::list);
+  T* L11 = reinterpret_cast<T*>(sm + Cfg::l11);  // by columns: l_ik at k SLD + i
+  T* Us = reinterpret_cast<T*>(sm + Cfg::us);
+  int* lab = reinterpret_cast<int*>(sm + Cfg::lab);
+  T* slab = reinterpret_cast<T*>(sm + slab_off);
+
+  const int q = (int)cluster_ctarank();
+  const int C = (int)cluster_nctarank();
+  const int tid = threadIdx.x, NT = blockDim.x;
+  const int lane = tid & 31, warp = tid >> 5, nw = NT >> 5;
   const int R = n - c0;
-  const int rpc_max = kLeafRowsTimesW / W;
-  const int C = cdiv(R, rpc_max);
-  const int rpc = cdiv(R, C);
-  const size_t smem = LeafSmem<T, W>::bytes(rpc, C);
-  auto kern = panel_leaf_kernel<T, W>;
+  const int rbeg = q * rpc;
+  const int rcnt = max(0, min(rpc, R - rbeg));
+  T* P = A + (long long)c0 * lda + c0;  // panel
+  T* Pm = P + (long long)rbeg * lda;    // this CTA's rows
+  constexpr int RPI = 32 / W;           // rows per warp access of the leaf's columns
+
+  if (tid == 0) {
+#pragma unroll
+    for (int b = 0; b < 3; ++b) mbar_init(&bars[b], 1);
+    fence_barrier_init();
+    if (q == 0) plan[0] = 0;
+  }
+
+  // logical row of each of this thread's rows (row s NT + tid of the CTA)
+  int lr[RPT];
+#pragma unroll
+  for (int s = 0; s < RPT; ++s) {
+    const int r = s * NT + tid;
+    lr[s] = r < rcnt ? rbeg + r : -1;  // -1: no row here, never active
+  }
+  // first leaf through the slab (whole rows per access)
+  {
+    const int w0 = min(W, pw);
+#pragma unroll 8
+    for (int r = warp * RPI + lane / W; r < rcnt; r += nw * RPI) {
+      const int c = lane % W;
+      slab[r * SLD + c] = c < w0 ? Pm[(long long)r * lda + c] : T(0);
+    }
+  }
+  __syncthreads();
+  cluster_sync_all();  // every CTA's barriers exist before anyone pushes into them
+
+  // this thread's part of a candidate's way to the other CTAs: chunk pch of
+  // the message to CTA pd (C MSG_CHUNKS <= 96 threads have one)
+  const int pd = tid / Cfg::MSG_CHUNKS, pch = tid % Cfg::MSG_CHUNKS;
+  const uint32_t push_dst = pd < C ? dsmem_map(cand + q, pd) + pch * 16 : 0u;
+  const uint32_t push_bar = pd < C ? dsmem_map(bars, pd) : 0u;
+
+  bool timed_out = false;
+  bool arrived = false;  // a cluster barrier arrival is outstanding (in-panel updates published)
+  // Row of the CTA (or -1) whose columns outside the current micro-panel this
+  // warp still has to send as pivot row j: its finished columns and its z, both
+  // in the slab, become row j of zrow in every CTA.
+  int zpush = -1;
+  auto send_z = [&](int j, int m0) {
+    if constexpr (ZW > 0) {
+      if (zpush >= 0) {  // uniform in the warp
+        __syncwarp();
+        constexpr int ZCH = ZW / V;  // 16-byte chunks
+        const T* sr = slab + zpush * SLD;
+        for (int e = lane; e < C * ZCH; e += 32) {
+          const int d = e / ZCH, c = (e % ZCH) * V;
+          const uint4 v = *reinterpret_cast<const uint4*>(sr + (c < m0 ? c : c + MW));
+          T* dst = zrow + j * ZW + c;
+          if (C > 1)
+            st_async_16(dsmem_map(dst, d), dsmem_map(&bars[2], d), v.x, v.y, v.z, v.w);
+          else
+            *reinterpret_cast<uint4*>(dst) = v;
+        }
+        zpush = -1;
+      }
+    }
+  };
+  int step = 0;  // columns so far: message buffer step & 1, mbarrier phase (step >> 1) & 1
+  uint32_t zphase = 0;
+
+  for (int o = 0, leaf = 0; o < pw; o += W, ++leaf) {
+    const int w = min(W, pw - o);
+    const int nc = pw - o - w;  // panel columns right of this leaf
+    T* Pn = P + o + W;          // (the first of them)
+    int* pid = prow_id + (leaf & 1) * W;
+    T y[RPT][MW];                // the micro-panel, rotated: slot 0 is the current column
+    T z[RPT][ZW > 0 ? ZW : 1];   // the leaf's columns right of it
+#pragma unroll
+    for (int s = 0; s < RPT; ++s) {
+      const int r = s * NT + tid;
+      if (r < rcnt) {
+        vec_load<T, MW>(y[s], slab + r * SLD);
+        if constexpr (ZW > 0) vec_load<T, ZW>(z[s], slab + r * SLD + MW);
+      } else {
+#pragma unroll
+        for (int c = 0; c < MW; ++c) y[s][c] = T(0);
+#pragma unroll
+        for (int c = 0; c < ZW; ++c) z[s][c] = T(0);
+      }
+    }
+
+#pragma unroll 1
+    for (int m0 = 0; m0 < w; m0 += MW) {
+      const int wm = min(MW, w - m0);
+      if (ZW > 0 && C > 1 && tid == 0) mbar_arrive_expect_tx(&bars[2], (uint32_t)(wm * ZW * sizeof(T)));
+      // this thread's best candidate for the next column
+      Key bk = 0;
+      int bi = INT_MAX, bs = 0;
+      T xb = T(1);
+      auto consider = [&](int s, T v, int J) {
+        Key k = PivKey<T>::of(v);
+        if (k == 0 && lr[s] == J && v != v) k = PivKey<T>::kForced;
+        if (RPT == 1 || bi == INT_MAX || k > bk || (k == bk && lr[s] < bi)) { bk = k; bi = lr[s]; bs = s; xb = v; }
+      };
+#pragma unroll
+      for (int s = 0; s < RPT; ++s)
+        if (lr[s] >= o + m0) consider(s, y[s][0], o + m0);
+
+      // One column per step.  The loop stays rolled, the registers rotating
+      // instead: unrolled over the micro-panel every step fetched its
+      // instructions anew and took a third longer.
+#pragma unroll 1
+      for (int j = 0; j < wm; ++j, ++step) {
+        const int J = o + m0 + j;
+        const int par = step & 1;
+        // ---- the warp's candidate, staged; then the CTA's, by every warp ----
+        const T rc = PivKey<T>::rcp(xb);
+        const int wl = warp_winner(bk, bi);
+        Msg* wms = wmsg + par * 16;
+        if (lane == wl) {
+          Msg* out = wms + warp;
+          out->key = bk;
+          out->label = bi;
+          out->row = bs * NT + tid;
+          out->rcp = rc;
+#pragma unroll
+          for (int s = 0; s < RPT; ++s)
+            if (s == bs) vec_store<T, MW>(out->v, y[s]);
+        }
+        if (C > 1 && tid == 0) mbar_arrive_expect_tx(&bars[par], (uint32_t)(C * sizeof(Msg)));
+        __syncthreads();
+        const int wo = warp_winner(lane < nw ? wms[lane].key : Key(0), lane < nw ? wms[lane].label : INT_MAX);
+        const Msg* win = wms + wo;
+        int qw = 0;
+        if (C > 1) {
+          // ---- to every CTA; then the best of all ----
+          Msg* in = cand + par * kPanelCtas;
+          if (pd < C) {
+            const uint4 v = reinterpret_cast<const uint4*>(win)[pch];
+            st_async_16(push_dst + par * (uint32_t)(kPanelCtas * sizeof(Msg)), push_bar + par * 8u, v.x, v.y, v.z, v.w);
+          }
+          if (j > 0) send_z(j - 1, m0);
+          if (!timed_out && !mbar_wait_spin(&bars[par], (uint32_t)((step >> 1) & 1), status)) timed_out = true;
+          qw = warp_winner(lane < C ? in[lane].key : Key(0), lane < C ? in[lane].label : INT_MAX);
+          if (qw >= C) qw = 0;
+          win = in + qw;
+        } else if (j > 0) {
+          send_z(j - 1, m0);
+        }
+        // (row J itself is always a candidate, so some CTA wins; the fallback
+        // only keeps the indexing in bounds)
+        const int p = win->label == INT_MAX ? J : win->label;
+        const T rcp = win->rcp;
+        T u[MW];
+        vec_load<T, MW>(u, win->v);
+        const T piv = u[0];
+        const bool safe = PivKey<T>::safe(piv);
+        const bool owner = qw == q && warp == wo && lane == wl;
+        const int bs_out = bs;  // (the owner lane's row)
+        // ---- interchange labels; multipliers; the micro-panel; next scan ----
+        bk = 0;
+        bi = INT_MAX;
+#pragma unroll
+        for (int s = 0; s < RPT; ++s) {
+          if (lr[s] == p) lr[s] = J;
+          else if (lr[s] == J) lr[s] = p;
+          T m = y[s][0];
+          if (lr[s] > J) {
+            m = div_by(y[s][0], piv, rcp);
+            if (!safe) m = y[s][0] / piv;
+#pragma unroll
+            for (int c = 1; c < MW; ++c)
+              if (c < MW - j) y[s][c] = fma(-m, u[c], y[s][c]);
+            consider(s, y[s][1], J + 1);
+          }
+          __syncwarp();  // rejoin at once: split, the warp would run all that follows twice
+#pragma unroll
+          for (int c = 0; c + 1 < MW; ++c) y[s][c] = y[s][c + 1];
+          y[s][MW - 1] = m;
+        }
+        // ---- the pivot row's other columns: into the slab (this part of it is
+        //      rewritten later), from where they go out beside the next exchange ----
+        if constexpr (ZW > 0) {
+          if (qw == q && warp == wo) {  // uniform in the warp
+            if (owner) {
+              T* sr = slab + (bs_out * NT + tid) * SLD + m0 + MW;
+#pragma unroll
+              for (int s = 0; s < RPT; ++s)
+                if (s == bs_out) {
+#pragma unroll
+                  for (int g = 0; g < ZW; g += MW)
+                    if (g < ZW - m0) vec_store<T, MW>(sr + g, z[s] + g);
+                }
+            }
+            __syncwarp();
+            zpush = __shfl_sync(0xffffffffu, bs_out * NT + tid, wl);
+          }
+        }
+        // L11 and the pivot's place, for the solves; the swap list
+        if (warp == nw - 1) {
+          if (lane < j) L11[(m0 + lane) * SLD + m0 + j] = win->v[MW - j + lane];
+          if (lane == 0) {
+            pid[m0 + j] = min(max(qw * rpc + win->row, 0), R - 1);
+            if (q == 0) {
+              ipiv[c0 + J] = c0 + p;
+              if (piv == T(0)) atomicCAS(status + 1, 0, c0 + J + 1);
+            }
+          }
+        }
+        __syncwarp();
+        // The buffers of this parity are rewritten two columns later, behind
+        // a barrier (here) and a message (elsewhere) that follow these reads.
+      }
+#pragma unroll 1
+      for (int k = wm; k < MW; ++k) {  // a narrower micro-panel: finish the rotation
+#pragma unroll
+        for (int s = 0; s < RPT; ++s) {
+          const T m = y[s][0];
+#pragma unroll
+          for (int c = 0; c + 1 < MW; ++c) y[s][c] = y[s][c + 1];
+          y[s][MW - 1] = m;
+        }
+      }
+
+      __syncwarp();
+      if constexpr (ZW > 0) {
+        send_z(wm - 1, m0);
+        if (C > 1 && !timed_out && !mbar_wait(&bars[2], zphase, status)) timed_out = true;
+        zphase ^= 1u;
+        __syncwarp();
+      }
+#pragma unroll
+      for (int s = 0; s < RPT; ++s) {
+        const int r = s * NT + tid;
+        if (r < rcnt) {
+          vec_store<T, MW>(slab + r * SLD + m0, y[s]);
+          lab[r] = lr[s];
+        }
+      }
+      __syncwarp();
+      if (m0 == 0 && arrived) cluster_wait();  // every CTA's updates of the columns from here on are visible
+      __syncthreads();  // pivot rows, L11 and pid complete
+      if (m0 == 0 && arrived) {
+        // every CTA has read the A12 rows of the leaf before: its U12 can go to
+        // its (unmoved) rows
+        const int uc = pw - o;
+        const int* id = prow_id + ((leaf & 1) ^ 1) * W;
+        for (int k = warp; k < W; k += nw) {
+          const int r = id[k];
+          if (r >= rbeg && r < rbeg + rcnt)
+            for (int c = lane; c < uc; c += 32) P[(long long)r * lda + o + c] = Us[k * LDU + c];
+        }
+        arrived = false;
+        __syncthreads();
+      }
+      // A12 of these pivot rows on its way
+      for (int k = m0 + warp; nc > 0 && k < m0 + wm; k += nw) {
+        const T* src = Pn + (long long)pid[k] * lda;
+        for (int c = lane * V; c < nc; c += 32 * V) {
+          if (c + V <= nc) {
+            cp_async16(Us + k * LDU + c, src + c);
+          } else {
+#pragma unroll
+            for (int e = 0; e < V; ++e)
+              if (c + e < nc) Us[k * LDU + c + e] = __ldcg(src + c + e);
+          }
+        }
+      }
+      if constexpr (ZW > 0) {
+        const int zl = ZW - m0;  // leaf columns right of the micro-panel
+        if (warp == 0) {
+          // U = L^-1 Z on them, lane = column
+          if (lane < zl && wm == MW) {
+            T v[MW];
+#pragma unroll
+            for (int i = 0; i < MW; ++i) v[i] = zrow[i * ZW + m0 + lane];
+            unit_lower_solve<T, MW>(v, L11 + m0 * SLD + m0, SLD);
+#pragma unroll
+            for (int i = 0; i < MW; ++i) zrow[i * ZW + m0 + lane] = v[i];
+          }
+        } else if (warp == 1) {
+          // the pivot rows' finished columns complete L11
+          for (int c = lane; c < m0; c += 32)
+            for (int i = 0; i < wm; ++i) L11[c * SLD + m0 + i] = zrow[i * ZW + c];
+        }
+        __syncthreads();
+        if (zl > 0 && wm == MW) {
+          // rank-MW update of them: every row below, and pivot row i with the i rows above it
+          int cnt[RPT];
+          bool full = true;
+#pragma unroll
+          for (int s = 0; s < RPT; ++s) {
+            const int d = lr[s] - (o + m0);
+            cnt[s] = min(max(d, 0), MW);
+            full = full && (d >= MW || lr[s] < 0);
+          }
+          full = __all_sync(0xffffffffu, full);
+#pragma unroll
+          for (int g = 0; g < ZW; g += MW) {
+            if (g < zl) {
+#pragma unroll
+              for (int k = 0; k < MW; ++k) {
+                T uk[MW];
+                vec_load<T, MW>(uk, zrow + k * ZW + m0 + g);
+#pragma unroll
+                for (int s = 0; s < RPT; ++s)
+                  if (full || k < cnt[s]) {
+#pragma unroll
+                    for (int c = 0; c < MW; ++c) z[s][g + c] = fma(-y[s][k], uk[c], z[s][g + c]);
+                  }
+              }
+            }
+          }
+#pragma unroll
+          for (int s = 0; s < RPT; ++s) {
+#pragma unroll
+            for (int c = 0; c < MW; ++c) y[s][c] = z[s][c];
+#pragma unroll
+            for (int c = 0; c + MW < ZW; ++c) z[s][c] = z[s][c + MW];
+          }
+        }
+      }
+    }
+
+    // ---- the leaf's columns back to their rows in memory (rows finished in an
+    //      earlier leaf hold U12 entries there) ----
+#pragma unroll 8
+    for (int r = warp * RPI + lane / W; r < rcnt; r += nw * RPI) {
+      const int c = lane % W;
+      if (c < w && lab[r] >= o) Pm[(long long)r * lda + o + c] = slab[r * SLD + c];
+    }
+    if (nc <= 0) break;
+    cp_async_wait_all();
+    __syncthreads();
+    // ---- U12 = L11^-1 A12 (w = W here), in every CTA ----
+    if (tid < nc) {
+      T v[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) v[i] = Us[i * LDU + tid];
+      unit_lower_solve<T, W>(v, L11, SLD);
+#pragma unroll
+      for (int i = 0; i < W; ++i) Us[i * LDU + tid] = v[i];
+    }
+    __syncthreads();
+    // ---- own rows -= L21 U12 in blocks of 32 rows x BW columns over the
+    //      warps, the next leaf's columns last: they replace L21 in the slab ----
+    constexpr int BW = W < 8 ? 8 : W;
+    const int nrb = (rcnt + 31) / 32, ncb = (nc + BW - 1) / BW;
+    for (int t = warp; t < nrb * (ncb - 1); t += nw) {
+      const int r0 = t % nrb * 32, cb = 1 + t / nrb;
+      panel_update<T, W, SLD, LDU, BW>(slab, Us + cb * BW, lab, o + W, r0, rcnt,
+                                       Pn + (long long)rbeg * lda + cb * BW, lda, nc - cb * BW, false);
+    }
+    __syncthreads();
+    for (int t = warp; t < nrb; t += nw)
+      panel_update<T, W, SLD, LDU, BW>(slab, Us, lab, o + W, t * 32, rcnt, Pn + (long long)rbeg * lda, lda, nc, true);
+    __syncthreads();
+    cluster_arrive();
+    arrived = true;
+  }
+
+  // ---- the rows that change place: list them, then move the panel's own
+  //      columns, a share of the columns per CTA ----
+#pragma unroll
+  for (int s = 0; s < RPT; ++s) {
+    const int r = s * NT + tid;
+    if (r < rcnt && lr[s] != rbeg + r) {
+      const int at = atomicAdd(plan, 1);  // at most 2 pw rows move
+      if (at < kSwapPlanRows) {
+        plan[1 + at] = c0 + lr[s];
+        plan[1 + kSwapPlanRows + at] = c0 + rbeg + r;
+      }
+    }
+  }
+  __syncthreads();
+  cluster_sync_all();
+  const int m = min(__ldcg(plan), kSwapPlanRows);
+  if (m == 0) return;
+  for (int e = tid; e < 2 * kSwapPlanRows; e += NT) list[e] = (e & (kSwapPlanRows - 1)) < m ? __ldcg(plan + 1 + e) : 0;
+  __syncthreads();
+  // (per warp access 4 rows x 8 columns; gathered to the slab, then scattered)
+  const int cw = ((pw + C - 1) / C + 7) / 8 * 8, cbeg = q * cw, cend = min(pw, cbeg + cw);
+  const int per = Cfg::slab_elems(rpc) / (8 * m) * 8;  // columns per pass through the slab
+  const int nr4 = (m + 3) / 4;
+  for (int cp = cbeg; cp < cend; cp += per) {
+    const int units = nr4 * ((min(per, cend - cp) + 7) / 8);
+    for (int t0 = warp; t0 < units; t0 += 8 * nw) {
+      T v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int t = t0 + i * nw, g = t / nr4, r = (t - g * nr4) * 4 + (lane >> 3), c = cp + g * 8 + (lane & 7);
+        v[i] = t < units && r < m && c < cend ? __ldcg(A + (long long)list[kSwapPlanRows + r] * lda + c0 + c) : T(0);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int t = t0 + i * nw, g = t / nr4, r = (t - g * nr4) * 4 + (lane >> 3);
+        if (t < units && r < m) slab[(g * m + r) * 8 + (lane & 7)] = v[i];
+      }
+    }
+    __syncthreads();
+    for (int t = warp; t < units; t += nw) {
+      const int g = t / nr4, r = (t - g * nr4) * 4 + (lane >> 3), c = cp + g * 8 + (lane & 7);
+      if (r < m && c < cend) A[(long long)list[r] * lda + c0 + c] = slab[(g * m + r) * 8 + (lane & 7)];
+    }
+    __syncthreads();
+  }
+}
+
+// Shape of the panel kernel for `rows` rows: leaf width W and rows per thread
+// RPT (W RPT registers of row data per thread: the widest leaf that holds the
+// rows), threads per CTA NT and CTAs C.  Short panels are spread over the
+// whole cluster, down to 32 rows per CTA: the in-panel updates then run on
+// more SMs.  Idle warps of a short CTA share its solves and updates.
+struct PanelShape {
+  int W = 0, RPT = 0, NT = 0, C = 0, rpc = 0;
+};
+
+int max_cluster(Ctx& c);
+
+template <typename T>
+PanelShape panel_shape(Ctx& c, int rows) {
+  PanelShape p;
+  const long long cm = max_cluster(c);
+  constexpr bool f32 = sizeof(T) == 4;
+  for (int lv = 0; lv < 4 && !p.W; ++lv) {
+    const int rpt = 1 << lv;
+    if (rows > cm * kPanelThreads * rpt) continue;
+    p.RPT = rpt;
+    p.W = f32 ? (lv < 2 ? 32 : 64 >> lv) : 32 >> lv;
+  }
+  if (!p.W) return p;
+  p.C = (int)std::min<long long>(cm, cdiv(rows, p.RPT > 1 ? kPanelThreads * p.RPT : 32));
+  p.rpc = cdiv(cdiv(rows, p.C), 32) * 32;  // whole 32-row blocks
+  p.NT = p.RPT > 1 ? kPanelThreads : std::max(128, p.rpc);
+  return p;
+}
+
+template <typename T, int W, int RPT>
+int launch_panel(Ctx& c, const PanelShape& ps, T* A, long long lda, int n, int c0, int pw, int* ipiv, int* plan,
+                 cudaStream_t st) {
+  using Cfg = PanelCfg<T, W, RPT>;
+  auto kern = panel_lu_kernel<T, W, RPT>;
   static bool attr_set[kMaxDevices] = {};
   const int dev = ctx_device(c);
   if (!attr_set[dev]) {
     LM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)LeafSmem<T, W>::bytes(rpc_max, 1)));
+                                     (int)Cfg::bytes(kPanelThreads * RPT)));
     LM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     attr_set[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(C, 1, 1);
-  cfg.blockDim = dim3(kLeafThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = dim3(ps.C, 1, 1);
+  cfg.blockDim = dim3(ps.NT, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::bytes(ps.rpc);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.x = ps.C;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, A, lda, n, c0, w, rpc, pc0, pw, ipiv, ctx_status(c)));
+  LM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, A, lda, n, c0, pw, ps.rpc, (unsigned)Cfg::slab_off(ps.rpc), ipiv, plan,
+                                 ctx_status(c)));
   count_launch(1);
   return LM_OK;
 }
 
-// Largest cluster the device schedules for the leaf kernel (16 when allowed).
+int g_max_cluster[kMaxDevices] = {};
+
+// Largest cluster the device schedules for the panel kernel (16 when allowed).
 int max_cluster(Ctx& c) {
   const int dev = ctx_device(c);
   if (g_max_cluster[dev]) return g_max_cluster[dev];
   int best = 8;
-  auto kern = panel_leaf_kernel<double, 16>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)LeafSmem<double, 16>::bytes(kLeafRowsTimesW / 16, 1)) == cudaSuccess &&
+  using Cfg = PanelCfg<double, 16, 2>;
+  auto kern = panel_lu_kernel<double, 16, 2>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::bytes(kPanelThreads * 2)) ==
+          cudaSuccess &&
       cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(16, 1, 1);
-    cfg.blockDim = dim3(kLeafThreads, 1, 1);
-    cfg.dynamicSmemBytes = LeafSmem<double, 16>::bytes(kLeafRowsTimesW / 16, 16);
+    cfg.gridDim = dim3(kPanelCtas, 1, 1);
+    cfg.blockDim = dim3(kPanelThreads, 1, 1);
+    cfg.dynamicSmemBytes = Cfg::bytes(kPanelThreads * 2);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.x = kPanelCtas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters > 0) best = 16;
+    if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters > 0) best = kPanelCtas;
   }
   cudaGetLastError();
   g_max_cluster[dev] = best;
@@ -485,29 +865,36 @@ int max_cluster(Ctx& c) {
 
 }  // namespace
 
-int panel_leaf_max_width_for(Ctx& c, int rows) {
-  const long long cap = (long long)max_cluster(c) * kLeafRowsTimesW;  // rows * W per cluster
-  for (int W = 32; W >= 4; W >>= 1)
-    if ((long long)rows * W <= cap) return W;
-  return 0;
+template <typename T>
+int panel_ctas(Ctx& c, int rows) {
+  return panel_shape<T>(c, rows).C;
 }
 
 template <typename T>
-int panel_leaf(Ctx& c, T* A, long long lda, int n, int c0, int w, int pc0, int pw, int* ipiv, cudaStream_t st) {
-  if (w <= 0) return LM_OK;
-  const int R = n - c0;
-  const int wmax = panel_leaf_max_width_for(c, R);
-  if (w > wmax || w > 32) return LM_ERR_UNSUPPORTED;
-  // smallest compiled width that holds w
-  if (pw > 128 || pc0 > c0 || pc0 + pw < c0 + w) return LM_ERR_ARG;
-  if (w <= 4 && wmax >= 4) return launch_leaf<T, 4>(c, A, lda, n, c0, w, pc0, pw, ipiv, st);
-  if (w <= 8 && wmax >= 8) return launch_leaf<T, 8>(c, A, lda, n, c0, w, pc0, pw, ipiv, st);
-  if (w <= 16 && wmax >= 16) return launch_leaf<T, 16>(c, A, lda, n, c0, w, pc0, pw, ipiv, st);
-  return launch_leaf<T, 32>(c, A, lda, n, c0, w, pc0, pw, ipiv, st);
+int panel_lu(Ctx& c, T* A, long long lda, int n, int c0, int pw, int* ipiv, int* plan, cudaStream_t st) {
+  if (pw <= 0) return LM_OK;
+  if (pw > kPanelNB || c0 + pw > n) return LM_ERR_ARG;
+  if ((reinterpret_cast<uintptr_t>(A) & 15) || (lda * (int)sizeof(T)) % 16 || (c0 * (int)sizeof(T)) % 16)
+    return LM_ERR_ARG;
+  const PanelShape ps = panel_shape<T>(c, n - c0);
+  if constexpr (sizeof(T) == 8) {
+    if (ps.W == 32) return launch_panel<T, 32, 1>(c, ps, A, lda, n, c0, pw, ipiv, plan, st);
+    if (ps.W == 16) return launch_panel<T, 16, 2>(c, ps, A, lda, n, c0, pw, ipiv, plan, st);
+    if (ps.W == 8) return launch_panel<T, 8, 4>(c, ps, A, lda, n, c0, pw, ipiv, plan, st);
+    if (ps.W == 4) return launch_panel<T, 4, 8>(c, ps, A, lda, n, c0, pw, ipiv, plan, st);
+  } else {
+    if (ps.W == 32 && ps.RPT == 1) return launch_panel<T, 32, 1>(c, ps, A, lda, n, c0, pw, ipiv, plan, st);
+    if (ps.W == 32) return launch_panel<T, 32, 2>(c, ps, A, lda, n, c0, pw, ipiv, plan, st);
+    if (ps.W == 16) return launch_panel<T, 16, 4>(c, ps, A, lda, n, c0, pw, ipiv, plan, st);
+    if (ps.W == 8) return launch_panel<T, 8, 8>(c, ps, A, lda, n, c0, pw, ipiv, plan, st);
+  }
+  return LM_ERR_UNSUPPORTED;
 }
 
-template int panel_leaf<double>(Ctx&, double*, long long, int, int, int, int, int, int*, cudaStream_t);
-template int panel_leaf<float>(Ctx&, float*, long long, int, int, int, int, int, int*, cudaStream_t);
+template int panel_ctas<double>(Ctx&, int);
+template int panel_ctas<float>(Ctx&, int);
+template int panel_lu<double>(Ctx&, double*, long long, int, int, int, int*, int*, cudaStream_t);
+template int panel_lu<float>(Ctx&, float*, long long, int, int, int, int*, int*, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Cholesky of one diagonal block (w <= 128), by 32-column panels in shared memory.
