@@ -28,26 +28,78 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-__global__ void __launch_bounds__(256) gemv_exact_kernel(int m, int n, const double* __restrict__ A, long long lda,
-                                                         const double* __restrict__ x, double* __restrict__ y) {
-  const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long row = gt >> 2;
-  const int l = threadIdx.x & 3;
-  const bool ok = row < m;
-  const double* ar = A + (ok ? row : 0) * lda;
+// One warp per CTA, 8 rows: lane l of a quad carries accumulator l of its row.
+// What bounds it is the bytes in flight: the four chains of a row are serial, so
+// a thread that loads as it goes has 8 loads of 8 bytes out (1.3 TB/s).  Here
+// each warp keeps kGemvStages chunks of 8 x 64 elements on their way through
+// shared memory with cp.async (16 bytes each where rows start on 16 bytes, else
+// 8), 29 KB per warp and 7 warps per SM.  The row stride of 68 puts the 8 quads
+// of a warp on different banks.
+// 8192 x 8192: 420 us before, 105 us now (5.1 TB/s, 0.78 of the copy rate).
+constexpr int kGemvRows = 8, kGemvCols = 64, kGemvLd = kGemvCols + 4, kGemvStages = 6;
+constexpr size_t kGemvSmem = sizeof(double) * kGemvStages * (kGemvRows * kGemvLd + kGemvCols);
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async_ca(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+
+template <int V>  // elements per copy of A: 2 (16 bytes) or 1
+__global__ void __launch_bounds__(32) gemv_exact_kernel(int m, int n, const double* __restrict__ A, long long lda,
+                                                        const double* __restrict__ x, double* __restrict__ y) {
+  extern __shared__ __align__(16) double gsm[];
+  double* sx = gsm + kGemvStages * kGemvRows * kGemvLd;  // x, by stage
+  const int lane = threadIdx.x, l = lane & 3, r = lane >> 2;
+  const int row0 = blockIdx.x * kGemvRows;
+  const int rows = min(kGemvRows, m - row0);
+  const double* Ab = A + (long long)row0 * lda;
   const int n4 = n - n % 4;
+  const int chunks = (n4 + kGemvCols - 1) / kGemvCols;
+  auto fetch = [&](int c) {
+    if (c < chunks) {
+      const int j0 = c * kGemvCols, cols = min(kGemvCols, n4 - j0);
+      double* sa = gsm + (c % kGemvStages) * kGemvRows * kGemvLd;
+      double* xs = sx + (c % kGemvStages) * kGemvCols;
+#pragma unroll
+      for (int q = 0; q < kGemvCols; q += 32)
+        if (q + lane < cols) cp_async_ca<8>(xs + q + lane, x + j0 + q + lane);
+#pragma unroll
+      for (int rr = 0; rr < kGemvRows; ++rr)
+#pragma unroll
+        for (int q = 0; q < kGemvCols; q += 32 * V) {
+          const int cc = q + lane * V;  // (cols is a multiple of 4)
+          if (rr < rows && cc < cols) cp_async_ca<8 * V>(sa + rr * kGemvLd + cc, Ab + (long long)rr * lda + j0 + cc);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int c = 0; c < kGemvStages - 1; ++c) fetch(c);
   double acc = 0.0;
-#pragma unroll 8
-  for (int j = l; j < n4; j += 4) acc = fma(ar[j], x[j], acc);
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kGemvStages - 2) : "memory");
+    __syncwarp();  // every lane's copies of chunk c are in; chunk c - 1 has been read
+    fetch(c + kGemvStages - 1);
+    const double* sa = gsm + (c % kGemvStages) * kGemvRows * kGemvLd + r * kGemvLd + l;
+    const double* xs = sx + (c % kGemvStages) * kGemvCols + l;
+    const int steps = min(kGemvCols, n4 - c * kGemvCols) / 4;
+    if (steps == kGemvCols / 4) {
+#pragma unroll
+      for (int s = 0; s < kGemvCols / 4; ++s) acc = fma(sa[4 * s], xs[4 * s], acc);
+    } else {
+      for (int s = 0; s < steps; ++s) acc = fma(sa[4 * s], xs[4 * s], acc);
+    }
+  }
   __syncwarp();
   // lane 0 of the quad gathers the four accumulators in the reference's order
   const double a1 = __shfl_down_sync(kFull, acc, 1, 4);
   const double a2 = __shfl_down_sync(kFull, acc, 2, 4);
   const double a3 = __shfl_down_sync(kFull, acc, 3, 4);
-  if (ok && l == 0) {
+  if (r < rows && l == 0) {
+    const double* ar = Ab + (long long)r * lda;
     double s = __dadd_rn(__dadd_rn(__dadd_rn(acc, a1), a2), a3);
     for (int j = n4; j < n; ++j) s = __dadd_rn(s, __dmul_rn(ar[j], x[j]));
-    y[row] = s;
+    y[row0 + r] = s;
   }
 }
 
@@ -224,7 +276,11 @@ int grid_for(long long total, int per) { return (int)std::max<long long>(1, std:
 
 int dgemv_exact(int m, int n, const double* A, long long lda, const double* x, double* y, cudaStream_t st) {
   if (m <= 0) return LM_OK;
-  gemv_exact_kernel<<<(int)cdivll(4LL * m, 256), 256, 0, st>>>(m, n, A, lda, x, y);
+  const int grid = (int)cdivll(m, kGemvRows);
+  if ((reinterpret_cast<uintptr_t>(A) & 15) || (lda & 1))
+    gemv_exact_kernel<1><<<grid, 32, kGemvSmem, st>>>(m, n, A, lda, x, y);
+  else
+    gemv_exact_kernel<2><<<grid, 32, kGemvSmem, st>>>(m, n, A, lda, x, y);
   count_launch(1);
   LM_CUDA_TRY(cudaGetLastError());
   return LM_OK;
