@@ -1,117 +1,24 @@
 // Row interchanges, triangular block solves, copies and the FP64 residual.
 //
-// laswp      : the row-swap half of rawSwapRows (K.hs:1507-1537) applied to
-//              the columns outside the current panel, and applyPivotsForward
-//              (LU.hs:493-507) on right-hand sides.
-// trsm_left  : the w x w triangular block solves of the blocked factorisations
-//              and substitutions — rawTriSolvePanelTrail (LU.hs:364-407) for
-//              U12, and the diagonal blocks of rawForwardSubUnitPackedSIMD,
-//              rawBackSubPackedSIMD, rawForwardSubCholPackedSIMD and
-//              rawBackSubCholTPackedSIMD (K.hs:2205-2430).
+// laswp_*    : applyPivotsForward (LU.hs:493-507) on right-hand sides, as one
+//              composed permutation.
+// trsm_left  : the diagonal blocks of the substitutions with several right-hand
+//              sides (rawForwardSubUnitPackedSIMD, rawBackSubPackedSIMD,
+//              rawForwardSubCholPackedSIMD and rawBackSubCholTPackedSIMD,
+//              K.hs:2205-2430).
 // dresidual  : r = b - A x in FP64, the GEMV of matvecP / rawGemv
 //              (L2.hs:131-139, K.hs:119-134) on the refinement path.
 #include <climits>
 
 #include "common.cuh"
 #include "internal.h"
+#include "pivot.cuh"
 
 namespace lm {
 
 void count_launch(int n);
 
 namespace {
-
-// Row interchanges as one composed permutation.  The swaps ipiv[k0..k1)
-// (at most kSwapChunk of them) touch at most 2 * kSwapChunk rows.  Thread 0
-// replays them on row indices in shared memory (rows k0..k1-1 in fixed
-// slots, other pivot rows found through a small open-addressing table),
-// giving for every touched row r the row src(r) whose data ends up in it.
-// The CTA then gathers all sources of its 32-column block into shared memory
-// (coalesced along the columns, many independent loads per thread) and
-// scatters them to their rows.
-constexpr int kSwapChunk = 128;
-constexpr int kSwapThreads = 256;
-constexpr int kHash = 512;
-
-template <typename T>
-__global__ void __launch_bounds__(kSwapThreads) laswp_kernel(T* A, long long lda, int nrows,
-                                                             const int* __restrict__ ipiv, int k0, int k1, int ca0,
-                                                             int ca1, int cb0, int cb1, int* status) {
-  __shared__ int rows[2 * kSwapChunk];
-  __shared__ int src[2 * kSwapChunk];
-  __shared__ int piv[kSwapChunk];
-  __shared__ int hkey[kHash];
-  __shared__ short hval[kHash];
-  __shared__ int list_r[2 * kSwapChunk];
-  __shared__ int list_s[2 * kSwapChunk];
-  __shared__ int m_sh, mm_sh;
-  extern __shared__ __align__(16) unsigned char sm[];
-  T* stage = reinterpret_cast<T*>(sm);  // [2 * kSwapChunk][32]
-  const int tid = threadIdx.x;
-  const int cnt = k1 - k0;
-  for (int i = tid; i < kHash; i += kSwapThreads) hkey[i] = -1;
-  for (int i = tid; i < cnt; i += kSwapThreads) {
-    rows[i] = k0 + i;
-    src[i] = k0 + i;
-    piv[i] = __ldg(ipiv + k0 + i);
-  }
-  if (tid == 0) mm_sh = 0;
-  __syncthreads();
-  if (tid == 0) {
-    int m = cnt;
-    for (int q = 0; q < cnt; ++q) {
-      const int k = k0 + q;
-      const int p = piv[q];
-      if (p < 0 || p >= nrows) {  // a bad swap list: record it, treat as no swap
-        atomicCAS(status, 0, LM_DEVERR_BOUNDS);
-        continue;
-      }
-      if (p == k) continue;
-      int sp;
-      if (p >= k0 && p < k1) {
-        sp = p - k0;
-      } else {
-        unsigned h = ((unsigned)p * 2654435761u) & (kHash - 1);
-        while (hkey[h] != -1 && hkey[h] != p) h = (h + 1) & (kHash - 1);
-        if (hkey[h] == p) {
-          sp = hval[h];
-        } else {
-          hkey[h] = p;
-          hval[h] = (short)m;
-          rows[m] = p;
-          src[m] = p;
-          sp = m++;
-        }
-      }
-      const int t = src[q];
-      src[q] = src[sp];
-      src[sp] = t;
-    }
-    m_sh = m;
-  }
-  __syncthreads();
-  // compact to the rows that actually change
-  for (int i = tid; i < m_sh; i += kSwapThreads)
-    if (src[i] != rows[i]) {
-      const int at = atomicAdd(&mm_sh, 1);
-      list_r[at] = rows[i];
-      list_s[at] = src[i];
-    }
-  __syncthreads();
-  const int mm = mm_sh;
-  const int na = ca1 - ca0, ncols = na + (cb1 - cb0);
-  const int lane = tid & 31, warp = tid >> 5;
-  const int t = blockIdx.x * 32 + lane;
-  const bool active = t < ncols;
-  const int col = t < na ? ca0 + t : cb0 + (t - na);
-#pragma unroll 4
-  for (int i = warp; i < mm; i += kSwapThreads / 32)
-    if (active) stage[i * 32 + lane] = A[(long long)list_s[i] * lda + col];
-  __syncthreads();
-#pragma unroll 4
-  for (int i = warp; i < mm; i += kSwapThreads / 32)
-    if (active) A[(long long)list_r[i] * lda + col] = stage[i * 32 + lane];
-}
 
 // All interchanges ipiv[0..n) on a narrow block B (n x nrhs) at once:
 // W(i, :) = B(sigma(i), :) with sigma(i) = tau_0(tau_1(... tau_{n-1}(i))),
@@ -194,80 +101,82 @@ __global__ void gather_rows_kernel(const T* __restrict__ B, long long ldb, int n
   }
 }
 
-// op(Tri) X = B for one w x 32 column block of B per CTA (w <= 128).  The
-// triangle of op(Tri) is staged packed in shared memory (w(w+1)/2 entries,
-// so two CTAs fit per SM in FP64) together with the block.  Rows are solved
-// in 16-row blocks: warp 0 solves a diagonal block (lane = column,
-// sequential over its 16 rows), then all warps apply the block to the rows
-// still to be solved (a rank-16 update).  Two barriers per 16 rows.
-__device__ __forceinline__ int tri_idx(bool upper, int w, int i, int k) {
-  return upper ? i * w - (i * (i - 1)) / 2 + (k - i) : (i * (i + 1)) / 2 + k;
-}
+// op(Tri) X = B for 8 columns of B per CTA (w <= 128): the block solves of the
+// substitutions with more than a few right-hand sides.  One launch after the
+// other, so latency bounds it: op(Tri) is staged whole (row stride 129, so that
+// a warp reads a column of it without conflicts), a thread keeps its row of B
+// (4 of the 8 columns) in registers, and the rows are solved in blocks of 32:
+//   solve  : warp h takes column h of the block, lane = row (tri_sweep);
+//   update : every thread applies the 32 solved entries to its row.
+// w = 128 with 64 columns: 86 us before (16-row blocks solved by one warp that
+// read every operand of its serial sums from shared memory), 33 us now; with 16
+// columns of a Cholesky factor in L2 86 and 23 us.
+constexpr int kTrsmLd = 129, kTrsmCols = 8;
+constexpr size_t kTrsmSmem = sizeof(double) * (128 * kTrsmLd + 128 + 2 * 32 * kTrsmCols);
 
-template <typename T>
-__global__ void __launch_bounds__(256) trsm_left_kernel(const T* __restrict__ Tri, long long ldt, int w,
-                                                       int lower, int unit, int trans, T* B, long long ldb,
-                                                       int ncols) {
+__global__ void __launch_bounds__(256) trsm_left_kernel(const double* __restrict__ Tri, long long ldt, int w, int lower,
+                                                        int unit, int trans, double* B, long long ldb, int ncols) {
   extern __shared__ __align__(16) unsigned char sm[];
   const bool upper_op = (lower == 0) != (trans != 0);
-  T* Ts = reinterpret_cast<T*>(sm);
-  T* Bs = Ts + ((w * (w + 1) / 2 + 1) & ~1);  // w x 32, ld 33
-  const int c0 = blockIdx.x * 32;
-  const int nc = min(32, ncols - c0);
-#pragma unroll 8
-  for (int i = threadIdx.x; i < w * w; i += blockDim.x) {
-    const int r = i / w, c = i % w;
-    if (lower ? (c <= r) : (c >= r)) {
-      const int oi = trans ? c : r, ok = trans ? r : c;
-      Ts[tri_idx(upper_op, w, oi, ok)] = Tri[(long long)r * ldt + c];
+  double* Ts = reinterpret_cast<double*>(sm);
+  double* dr = Ts + 128 * kTrsmLd;  // reciprocals of the diagonal
+  double* Xs = dr + 128;            // [2][32][8] the block being solved, by parity
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c0 = blockIdx.x * kTrsmCols;
+  const int nc = min(kTrsmCols, ncols - c0);
+  const int row = tid & 127, cg = (tid >> 7) * 4;  // this thread's row and columns of B
+  double x[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) x[c] = row < w && cg + c < nc ? B[(long long)row * ldb + c0 + cg + c] : 0.0;
+#pragma unroll 16
+  for (int r = warp; r < w; r += 8) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = q * 32 + lane;
+      if (c < w && (lower ? c <= r : c >= r))
+        Ts[trans ? c * kTrsmLd + r : r * kTrsmLd + c] = __ldg(Tri + (long long)r * ldt + c);
     }
-  }
-#pragma unroll 8
-  for (int i = threadIdx.x; i < w * 32; i += blockDim.x) {
-    const int r = i >> 5, c = i & 31;
-    Bs[r * 33 + c] = (c < nc) ? B[(long long)r * ldb + c0 + c] : T(0);
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nwarps = blockDim.x >> 5;
-  const int nb = (w + 15) / 16;
+  if (!unit && tid < w) dr[tid] = 1.0 / Ts[tid * kTrsmLd + tid];  // (read after the next barrier)
+  const int nb = (w + 31) / 32;
   for (int bi = 0; bi < nb; ++bi) {
-    const int b = upper_op ? nb - 1 - bi : bi;
-    const int r0 = b * 16, r1 = min(r0 + 16, w);
-    if (warp == 0) {
-      if (!upper_op) {
-        for (int r = r0; r < r1; ++r) {
-          const T* trow = Ts + tri_idx(false, w, r, 0);
-          T x = Bs[r * 33 + lane];
-          for (int q = r0; q < r; ++q) x = fma(-trow[q], Bs[q * 33 + lane], x);
-          if (!unit) x = x / trow[r];
-          Bs[r * 33 + lane] = x;
-        }
-      } else {
-        for (int r = r1 - 1; r >= r0; --r) {
-          const T* trow = Ts + tri_idx(true, w, r, r) - r;  // trow[q] = op(T)(r, q), q >= r
-          T x = Bs[r * 33 + lane];
-          for (int q = r + 1; q < r1; ++q) x = fma(-trow[q], Bs[q * 33 + lane], x);
-          if (!unit) x = x / trow[r];
-          Bs[r * 33 + lane] = x;
-        }
+    const int r0 = (upper_op ? nb - 1 - bi : bi) * 32, bw = min(32, w - r0);
+    double* X = Xs + (bi & 1) * 32 * kTrsmCols;
+    if (row >= r0 && row < r0 + 32) {  // uniform in the warp
+#pragma unroll
+      for (int c = 0; c < 4; ++c) X[(row - r0) * kTrsmCols + cg + c] = x[c];
+    }
+    __syncthreads();
+    if (warp < nc) {
+      double y = X[lane * kTrsmCols + warp];
+      const bool in = lane < bw;
+      const double* trow = Ts + (in ? r0 + lane : r0) * kTrsmLd + r0;
+      const double d = unit || !in ? 1.0 : trow[lane], rd = unit || !in ? 1.0 : dr[r0 + lane];
+      y = tri_sweep<double, 32>(y, trow, d, rd, lane, bw, !upper_op, unit != 0);
+      if (in) X[lane * kTrsmCols + warp] = y;
+    }
+    __syncthreads();
+    if (row >= r0 && row < r0 + 32) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) x[c] = X[(row - r0) * kTrsmCols + cg + c];
+    } else if (row < w && (upper_op ? row < r0 : row > r0)) {
+      const double* trow = Ts + row * kTrsmLd + r0;
+#pragma unroll 8
+      for (int k = 0; k < bw; ++k) {
+        const double t = trow[k];
+        const double2 a = *reinterpret_cast<const double2*>(X + k * kTrsmCols + cg);
+        const double2 b = *reinterpret_cast<const double2*>(X + k * kTrsmCols + cg + 2);
+        x[0] = fma(-t, a.x, x[0]);
+        x[1] = fma(-t, a.y, x[1]);
+        x[2] = fma(-t, b.x, x[2]);
+        x[3] = fma(-t, b.y, x[3]);
       }
     }
-    __syncthreads();
-    // rank-(r1-r0) update of the unsolved rows
-    const int u0 = upper_op ? 0 : r1, u1 = upper_op ? r0 : w;
-    for (int i = u0 + warp; i < u1; i += nwarps) {
-      const T* trow = upper_op ? Ts + tri_idx(true, w, i, i) - i : Ts + tri_idx(false, w, i, 0);
-      T acc = Bs[i * 33 + lane];
-      for (int q = r0; q < r1; ++q) acc = fma(-trow[q], Bs[q * 33 + lane], acc);
-      Bs[i * 33 + lane] = acc;
-    }
-    __syncthreads();
   }
-  for (int i = threadIdx.x; i < w * 32; i += blockDim.x) {
-    const int r = i >> 5, c = i & 31;
-    if (c < nc) B[(long long)r * ldb + c0 + c] = Bs[r * 33 + c];
-  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if (row < w && cg + c < nc) B[(long long)row * ldb + c0 + cg + c] = x[c];
 }
 
 template <typename T>
@@ -340,30 +249,6 @@ int grid_for(long long total, int threads, int sms) {
 
 }  // namespace
 
-template <typename T>
-int laswp(T* A, long long lda, int nrows, const int* ipiv, int k0, int k1, int ca0, int ca1, int cb0, int cb1,
-          int* status, cudaStream_t st) {
-  ca1 = std::max(ca0, ca1);
-  cb1 = std::max(cb0, cb1);
-  const int cols = (ca1 - ca0) + (cb1 - cb0);
-  if (cols == 0 || k1 <= k0) return LM_OK;
-  const size_t smem = sizeof(T) * 2 * kSwapChunk * 32;
-  static bool attr_set[kMaxDevices] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set[dev]) {
-    LM_CUDA_TRY(cudaFuncSetAttribute(laswp_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set[dev] = true;
-  }
-  for (int s0 = k0; s0 < k1; s0 += kSwapChunk) {
-    const int s1 = std::min(k1, s0 + kSwapChunk);
-    laswp_kernel<T><<<cdiv(cols, 32), kSwapThreads, smem, st>>>(A, lda, nrows, ipiv, s0, s1, ca0, ca1, cb0, cb1, status);
-    count_launch(1);
-    LM_CUDA_TRY(cudaGetLastError());
-  }
-  return LM_OK;
-}
-
 int perm_from_swaps(const int* ipiv, int n, int* perm, int* status, cudaStream_t st) {
   if (n <= 0) return LM_OK;
   perm_from_swaps_kernel<<<cdiv(n, 128), 128, 0, st>>>(ipiv, n, perm, status);
@@ -392,22 +277,19 @@ int laswp_narrow(T* B, long long ldb, int n, int nrhs, const int* ipiv, T* W, in
   return copy2d<T>(B, ldb, W, nrhs, n, nrhs, st);
 }
 
-template <typename T>
-int trsm_left(const T* Tri, long long ldt, int w, bool lower, bool unit, bool trans, T* B, long long ldb,
+int trsm_left(const double* Tri, long long ldt, int w, bool lower, bool unit, bool trans, double* B, long long ldb,
               int ncols, cudaStream_t st) {
   if (w <= 0 || ncols <= 0) return LM_OK;
   if (w > 128) return LM_ERR_ARG;
-  const size_t smem = sizeof(T) * ((size_t)((w * (w + 1) / 2 + 1) & ~1) + (size_t)w * 33);
   static bool attr_set[kMaxDevices] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    LM_CUDA_TRY(cudaFuncSetAttribute(trsm_left_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(sizeof(T) * (128 * 129 / 2 + 1 + 128 * 33))));
+    LM_CUDA_TRY(cudaFuncSetAttribute(trsm_left_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
     attr_set[dev] = true;
   }
-  trsm_left_kernel<T><<<cdiv(ncols, 32), 256, smem, st>>>(Tri, ldt, w, lower ? 1 : 0, unit ? 1 : 0,
-                                                          trans ? 1 : 0, B, ldb, ncols);
+  trsm_left_kernel<<<cdiv(ncols, kTrsmCols), 256, kTrsmSmem, st>>>(Tri, ldt, w, lower ? 1 : 0, unit ? 1 : 0,
+                                                                   trans ? 1 : 0, B, ldb, ncols);
   count_launch(1);
   LM_CUDA_TRY(cudaGetLastError());
   return LM_OK;
@@ -474,16 +356,10 @@ int dresidual(Ctx& c, int n, int nrhs, const double* A, long long lda, const dou
   return dgemm(c, d, st);
 }
 
-template int laswp<double>(double*, long long, int, const int*, int, int, int, int, int, int, int*, cudaStream_t);
-template int laswp<float>(float*, long long, int, const int*, int, int, int, int, int, int, int*, cudaStream_t);
 template int laswp_narrow<double>(double*, long long, int, int, const int*, double*, int*, cudaStream_t);
 template int laswp_narrow<float>(float*, long long, int, int, const int*, float*, int*, cudaStream_t);
 template int laswp_perm<double>(double*, long long, int, int, const int*, double*, cudaStream_t);
 template int laswp_perm<float>(float*, long long, int, int, const int*, float*, cudaStream_t);
-template int trsm_left<double>(const double*, long long, int, bool, bool, bool, double*, long long, int,
-                               cudaStream_t);
-template int trsm_left<float>(const float*, long long, int, bool, bool, bool, float*, long long, int,
-                              cudaStream_t);
 template int copy2d<double>(double*, long long, const double*, long long, int, int, cudaStream_t);
 template int copy2d<float>(float*, long long, const float*, long long, int, int, cudaStream_t);
 template int set_identity<double>(double*, long long, int, int, cudaStream_t);

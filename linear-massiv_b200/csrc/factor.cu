@@ -275,23 +275,29 @@ int dgetrf_nopiv(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
 namespace {
 
 // Copy to even-stride, 16-byte aligned buffers when the caller's are not
-// (TMA row alignment); returns the buffers to use.
+// (TMA row alignment); returns the buffers to use.  With `perm_ints` the
+// workspace also holds the right-hand side's interchanges: that many ints,
+// then n x nrhs doubles.
 struct SolveBufs {
   const double* M;
   long long ldm;
   double* X;
   long long ldx;
   bool copied_x;
+  int* perm;
+  double* W;
 };
 
-int solve_bufs(Ctx& c, int n, int nrhs, const double* M, long long ldm, double* B, long long ldb,
+int solve_bufs(Ctx& c, int n, int nrhs, const double* M, long long ldm, double* B, long long ldb, int perm_ints,
                SolveBufs& sb, cudaStream_t st) {
-  sb.M = M; sb.ldm = ldm; sb.X = B; sb.ldx = ldb; sb.copied_x = false;
+  sb.M = M; sb.ldm = ldm; sb.X = B; sb.ldx = ldb; sb.copied_x = false; sb.perm = nullptr; sb.W = nullptr;
   const bool m_ok = !(reinterpret_cast<uintptr_t>(M) & 15) && !(ldm & 1);
   const bool x_ok = !(reinterpret_cast<uintptr_t>(B) & 15) && !(ldb & 1);
   const long long ldm2 = m_ok ? 0 : (n + 7) / 8 * 8;
   const long long ldx2 = x_ok ? 0 : (nrhs + 7) / 8 * 8;
-  const size_t bytes = sizeof(double) * ((size_t)n * ldm2 + (size_t)n * ldx2);
+  const size_t perm_doubles = (size_t)(perm_ints + 7) / 8 * 4;
+  const size_t bytes = sizeof(double) * ((size_t)n * ldm2 + (size_t)n * ldx2 +
+                                         (perm_ints ? perm_doubles + (size_t)n * nrhs : 0));
   if (bytes == 0) return LM_OK;
   void* ws = nullptr;
   LM_TRY(ctx_workspace(c, 2, bytes, &ws));
@@ -304,6 +310,11 @@ int solve_bufs(Ctx& c, int n, int nrhs, const double* M, long long ldm, double* 
   if (!x_ok) {
     LM_TRY(copy2d<double>(p, ldx2, B, ldb, n, nrhs, st));
     sb.X = p; sb.ldx = ldx2; sb.copied_x = true;
+    p += (size_t)n * ldx2;
+  }
+  if (perm_ints) {
+    sb.perm = reinterpret_cast<int*>(p);
+    sb.W = p + perm_doubles;
   }
   return LM_OK;
 }
@@ -316,7 +327,7 @@ int forward_blocked(Ctx& c, int n, int nrhs, const double* M, long long ldm, boo
     const double* Mii = M + (long long)i0 * ldm + i0;
     {
       Prof p(c, kPhaseTrsm, (double)w * w * nrhs, 8.0 * ((double)w * w / 2 + 2.0 * w * nrhs), st);
-      LM_TRY(trsm_left<double>(Mii, ldm, w, true, unit, false, X + (long long)i0 * ldx, ldx, nrhs, st));
+      LM_TRY(trsm_left(Mii, ldm, w, true, unit, false, X + (long long)i0 * ldx, ldx, nrhs, st));
     }
     if (i0 + w < n) {
       GemmDesc d;
@@ -347,11 +358,14 @@ int dgetrs(Ctx& c, int n, int nrhs, const double* LU, long long lda, const int* 
     return trsv_lu<double>(LU, lda, n, nrhs, nullptr, nullptr, B, ldb, static_cast<int*>(ws), ctx_status(c), st);
   }
   SolveBufs sb;
-  LM_TRY(solve_bufs(c, n, nrhs, LU, lda, B, ldb, sb, st));
-  // P b (applyPivotsForward, LU.hs:493-507)
+  LM_TRY(solve_bufs(c, n, nrhs, LU, lda, B, ldb, n, sb, st));
+  // P b (applyPivotsForward, LU.hs:493-507): the swaps composed once, then a
+  // gather (n = 8192, 64 columns: 2.2 ms as 64 launches of 128 swaps each, 0.12 ms
+  // now)
   {
     Prof p(c, kPhaseSwap, 0.0, 32.0 * n * nrhs, st);
-    LM_TRY(laswp<double>(sb.X, sb.ldx, n, ipiv, 0, n, 0, nrhs, 0, 0, ctx_status(c), st));
+    LM_TRY(perm_from_swaps(ipiv, n, sb.perm, ctx_status(c), st));
+    LM_TRY(laswp_perm<double>(sb.X, sb.ldx, n, nrhs, sb.perm, sb.W, st));
   }
   LM_TRY(forward_blocked(c, n, nrhs, sb.M, sb.ldm, true, sb.X, sb.ldx, st));
   const int nblk = (n + kNB - 1) / kNB;
@@ -361,7 +375,7 @@ int dgetrs(Ctx& c, int n, int nrhs, const double* LU, long long lda, const int* 
     const double* Uii = sb.M + (long long)i0 * sb.ldm + i0;
     {
       Prof p(c, kPhaseTrsm, (double)w * w * nrhs, 8.0 * ((double)w * w / 2 + 2.0 * w * nrhs), st);
-      LM_TRY(trsm_left<double>(Uii, sb.ldm, w, false, false, false, sb.X + (long long)i0 * sb.ldx, sb.ldx, nrhs,
+      LM_TRY(trsm_left(Uii, sb.ldm, w, false, false, false, sb.X + (long long)i0 * sb.ldx, sb.ldx, nrhs,
                                st));
     }
     if (i0 > 0) {
@@ -396,7 +410,7 @@ int dpotrs(Ctx& c, int n, int nrhs, const double* G, long long lda, double* B, l
     return trsv_lu<double>(P, ldp, n, nrhs, nullptr, nullptr, B, ldb, sync, ctx_status(c), st, nullptr, true, false);
   }
   SolveBufs sb;
-  LM_TRY(solve_bufs(c, n, nrhs, G, lda, B, ldb, sb, st));
+  LM_TRY(solve_bufs(c, n, nrhs, G, lda, B, ldb, 0, sb, st));
   LM_TRY(forward_blocked(c, n, nrhs, sb.M, sb.ldm, false, sb.X, sb.ldx, st));
   // G^T x = y, bottom-up; the off-diagonal update uses G's row block transposed.
   const int nblk = (n + kNB - 1) / kNB;
@@ -406,7 +420,7 @@ int dpotrs(Ctx& c, int n, int nrhs, const double* G, long long lda, double* B, l
     const double* Gii = sb.M + (long long)i0 * sb.ldm + i0;
     {
       Prof p(c, kPhaseTrsm, (double)w * w * nrhs, 8.0 * ((double)w * w / 2 + 2.0 * w * nrhs), st);
-      LM_TRY(trsm_left<double>(Gii, sb.ldm, w, true, false, true, sb.X + (long long)i0 * sb.ldx, sb.ldx, nrhs,
+      LM_TRY(trsm_left(Gii, sb.ldm, w, true, false, true, sb.X + (long long)i0 * sb.ldx, sb.ldx, nrhs,
                                st));
     }
     if (i0 > 0) {

@@ -96,13 +96,6 @@ struct GemmDesc {
 int dgemm(Ctx& c, const GemmDesc& d, cudaStream_t st);
 
 // --- shared kernels (blas_aux.cu) --------------------------------------------
-// Apply row interchanges ipiv[k0..k1) in order (row s <-> row ipiv[s]) to the
-// columns [ca0, ca1) and [cb0, cb1) of A (nrows rows).  A pivot row outside
-// [0, nrows) is skipped and recorded as LM_DEVERR_BOUNDS in status[0].
-template <typename T>
-int laswp(T* A, long long lda, int nrows, const int* ipiv, int k0, int k1, int ca0, int ca1, int cb0, int cb1,
-          int* status, cudaStream_t st);
-
 // Row plan of one panel's interchanges: [0] the number of rows that change
 // place (at most kSwapPlanRows), then their destination rows, then (from
 // 1 + kSwapPlanRows) the rows they come from.
@@ -130,9 +123,8 @@ int laswp_perm(T* B, long long ldb, int n, int nrhs, const int* perm, T* W, cuda
 // In-place triangular solve with a w x w block (w <= 128) of Tri (ldt) on the
 // w x ncols block B (ldb):  op(Tri) X = B.
 //   lower/unit describe Tri as stored; trans solves with Tri^T.
-template <typename T>
-int trsm_left(const T* Tri, long long ldt, int w, bool lower, bool unit, bool trans, T* B,
-              long long ldb, int ncols, cudaStream_t st);
+int trsm_left(const double* Tri, long long ldt, int w, bool lower, bool unit, bool trans, double* B, long long ldb,
+              int ncols, cudaStream_t st);
 
 // Inverse of a lower-triangular block of order w <= 128 (diag.cu): Xout
 // (w x w, ldx) <- inv(L) with zeros above the diagonal; `unit` ignores the
@@ -218,8 +210,6 @@ int potrf_block(Ctx& c, T* A, long long lda, int w, int base, cudaStream_t st);
 // substitutions, FP64 refinement.  `factor_runner` runs the factorisation
 // body (so the caller can capture it into a CUDA graph).
 int sgetrf(Ctx& c, int n, float* A, long long lda, int* ipiv, cudaStream_t st, int prec = LM_IR_PREC_TF32X3);
-int sgetrs(Ctx& c, int n, int nrhs, const float* LU, long long lda, const int* ipiv, float* X, long long ldx,
-           cudaStream_t st);
 // Runs a fixed launch sequence tagged "factor" or "iter" (the caller maps the
 // tag and the solve's buffers to a CUDA-graph key, or runs it eagerly).
 using IrRunner = std::function<int(const char* tag, const std::function<int(cudaStream_t)>& body)>;

@@ -136,35 +136,6 @@ __global__ void transpose_to_bf16_kernel(__nv_bfloat16* dst, long long ldd, cons
   }
 }
 
-// X[m x nrhs] -= M[m x k] * Y[k x nrhs] in FP32 (exact fp32 FMAs), one warp per
-// row, nrhs <= 64 (the right-hand-side updates of the FP32 substitutions).
-__global__ void sgemm_rhs_kernel(int m, int k, int nrhs, const float* __restrict__ M, long long ldm,
-                                 const float* __restrict__ Y, long long ldy, float* X, long long ldx) {
-  const int warps = blockDim.x >> 5;
-  const int row = blockIdx.x * warps + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= m) return;
-  const float* mr = M + (long long)row * ldm;
-  for (int c0 = 0; c0 < nrhs; c0 += 8) {
-    float acc[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) acc[c] = 0.f;
-    for (int kk = lane; kk < k; kk += 32) {
-      const float a = mr[kk];
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        if (c0 + c < nrhs) acc[c] = fmaf(a, Y[(long long)kk * ldy + c0 + c], acc[c]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-    if (lane == 0)
-      for (int c = 0; c < 8 && c0 + c < nrhs; ++c) X[(long long)row * ldx + c0 + c] -= acc[c];
-  }
-}
-
 // X (FP64) += D (FP32); R (FP32) <- fl32(Rd) helpers.
 __global__ void add_s2d_kernel(double* X, long long ldx, const float* D, long long ldd, int rows, int cols) {
   const long long total = (long long)rows * cols;
@@ -314,49 +285,6 @@ int sgetrf(Ctx& c, int n, float* A, long long lda, int* ipiv, cudaStream_t st, i
       LM_CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
     else
       LM_TRY(panel(nx, st));
-  }
-  return LM_OK;
-}
-
-// Solve with the FP32 factors: X (n x nrhs, FP32, ldx) overwritten.
-int sgetrs(Ctx& c, int n, int nrhs, const float* LU, long long lda, const int* ipiv, float* X, long long ldx,
-           cudaStream_t st) {
-  {
-    Prof p(c, kPhaseSwap, 0.0, 16.0 * n * nrhs, st);
-    LM_TRY(laswp<float>(X, ldx, n, ipiv, 0, n, 0, nrhs, 0, 0, ctx_status(c), st));
-  }
-  for (int i0 = 0; i0 < n; i0 += kNB) {
-    const int w = std::min(kNB, n - i0);
-    const float* Lii = LU + (long long)i0 * lda + i0;
-    {
-      Prof p(c, kPhaseTrsm, (double)w * w * nrhs, 4.0 * ((double)w * w / 2 + 2.0 * w * nrhs), st);
-      LM_TRY(trsm_left<float>(Lii, lda, w, true, true, false, X + (long long)i0 * ldx, ldx, nrhs, st));
-    }
-    if (i0 + w < n) {
-      const int m = n - i0 - w;
-      Prof p(c, kPhaseGemm, 2.0 * m * w * nrhs, 4.0 * (double)m * w, st);
-      sgemm_rhs_kernel<<<cdiv(m, 8), 256, 0, st>>>(m, w, nrhs, Lii + (long long)w * lda, lda,
-                                                   X + (long long)i0 * ldx, ldx, X + (long long)(i0 + w) * ldx, ldx);
-      count_launch(1);
-      LM_CUDA_TRY(cudaGetLastError());
-    }
-  }
-  const int nblk = (n + kNB - 1) / kNB;
-  for (int b = nblk - 1; b >= 0; --b) {
-    const int i0 = b * kNB;
-    const int w = std::min(kNB, n - i0);
-    const float* Uii = LU + (long long)i0 * lda + i0;
-    {
-      Prof p(c, kPhaseTrsm, (double)w * w * nrhs, 4.0 * ((double)w * w / 2 + 2.0 * w * nrhs), st);
-      LM_TRY(trsm_left<float>(Uii, lda, w, false, false, false, X + (long long)i0 * ldx, ldx, nrhs, st));
-    }
-    if (i0 > 0) {
-      Prof p(c, kPhaseGemm, 2.0 * i0 * w * nrhs, 4.0 * (double)i0 * w, st);
-      sgemm_rhs_kernel<<<cdiv(i0, 8), 256, 0, st>>>(i0, w, nrhs, LU + i0, lda, X + (long long)i0 * ldx, ldx, X,
-                                                    ldx);
-      count_launch(1);
-      LM_CUDA_TRY(cudaGetLastError());
-    }
   }
   return LM_OK;
 }

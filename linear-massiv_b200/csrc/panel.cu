@@ -39,6 +39,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "pivot.cuh"
 
 namespace lm {
 
@@ -49,79 +50,6 @@ namespace {
 constexpr int kPanelNB = 128;      // widest panel
 constexpr int kPanelThreads = 512; // most threads per CTA (one row of the leaf each, times RPT)
 constexpr int kPanelCtas = 16;     // largest cluster
-
-// The pivot order of the reference's scan (strict '>' from row j down): the
-// larger |a| wins, the lower row on ties, NaN never wins.  |a| becomes an
-// integer key in that order, its IEEE bits, so that a warp reduces it with
-// redux.sync.  NaN gets the key of zero: row j, which has the lowest label, is
-// always among the candidates, so neither ever beats it.  Row j with a NaN
-// a_jj stays the pivot (the reference scan starts at row j and NaN never
-// compares greater): kForced beats every other key.
-template <typename T>
-struct PivKey;
-template <>
-struct PivKey<double> {
-  using K = unsigned long long;
-  static constexpr K kForced = ~0ull;
-  __device__ static K of(double x) {
-    const K u = (K)__double_as_longlong(x) & 0x7fffffffffffffffull;
-    return u > 0x7ff0000000000000ull ? 0ull : u;
-  }
-  // the reciprocal of a pivot in this range and the remainders formed with
-  // it neither overflow nor lose bits to underflow
-  __device__ static bool safe(double p) { const double a = fabs(p); return a > 0x1p-500 && a < 0x1p500; }
-  // 1 / p to about an ulp: the hardware estimate and two Newton steps
-  __device__ static double rcp(double p) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(p));
-    r = fma(r, fma(-p, r, 1.0), r);
-    return fma(r, fma(-p, r, 1.0), r);
-  }
-};
-template <>
-struct PivKey<float> {
-  using K = unsigned;
-  static constexpr K kForced = ~0u;
-  __device__ static K of(float x) {
-    const K u = __float_as_uint(x) & 0x7fffffffu;
-    return u > 0x7f800000u ? 0u : u;
-  }
-  __device__ static bool safe(float p) { const float a = fabsf(p); return a > 0x1p-60f && a < 0x1p60f; }
-  __device__ static float rcp(float p) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(p));
-    return fmaf(r, fmaf(-p, r, 1.f), r);
-  }
-};
-
-// Lane (the same in every lane) holding the warp's best (key, label): the
-// largest key, then the lowest label.  Lanes without a candidate pass key 0
-// and label INT_MAX.  Usually one redux.sync and one vote: the later rounds
-// run only when several lanes share the leading bits.
-__device__ __forceinline__ int warp_winner(unsigned key, int label) {
-  __syncwarp();  // reconverge: a split warp would serialise every *_sync below
-  unsigned b = __ballot_sync(0xffffffffu, key == __reduce_max_sync(0xffffffffu, key));
-  if (b & (b - 1)) {
-    const unsigned l = (b >> (threadIdx.x & 31)) & 1 ? (unsigned)label : 0xffffffffu;
-    b = __ballot_sync(0xffffffffu, l == __reduce_min_sync(0xffffffffu, l));
-  }
-  return __ffs(b) - 1;
-}
-__device__ __forceinline__ int warp_winner(unsigned long long key, int label) {
-  __syncwarp();
-  const unsigned hi = (unsigned)(key >> 32);
-  unsigned b = __ballot_sync(0xffffffffu, hi == __reduce_max_sync(0xffffffffu, hi));
-  if (b & (b - 1)) {
-    const int lane = threadIdx.x & 31;
-    const unsigned lo = (b >> lane) & 1 ? (unsigned)key : 0u;
-    b &= __ballot_sync(0xffffffffu, lo == __reduce_max_sync(0xffffffffu, lo));
-    if (b & (b - 1)) {
-      const unsigned l = (b >> lane) & 1 ? (unsigned)label : 0xffffffffu;
-      b &= __ballot_sync(0xffffffffu, l == __reduce_min_sync(0xffffffffu, l));
-    }
-  }
-  return __ffs(b) - 1;
-}
 
 // The candidate that each CTA sends to every CTA of the cluster, once per
 // column: 16-byte chunks, header then the micro-panel's part of the row in
@@ -276,14 +204,6 @@ __device__ __forceinline__ void panel_update(T* slab, const T* U, const int* lab
       }
     }
   }
-}
-
-// x / p for a pivot p whose correctly rounded reciprocal is r: the quotient
-// estimate x r corrected once by its exact remainder (Markstein 1990).
-template <typename T>
-__device__ __forceinline__ T div_by(T x, T p, T r) {
-  const T q = x * r;
-  return fma(fma(-p, q, x), r, q);
 }
 
 // N elements between a thread's registers and 16-byte aligned shared memory.
