@@ -298,8 +298,7 @@ int run_graphed(Ctx& c, const std::string& key0, F&& body) {
   return LM_OK;
 }
 
-int dpotrf_borrowed(int device, int num_sms, cudaStream_t st, int n, double* A, long long lda, int* d_status,
-                    void* scratch, size_t scratch_bytes) {
+int dpotrf_borrowed(int device, int num_sms, cudaStream_t st, int n, double* A, long long lda, int* d_status) {
   Ctx c;
   c.device = device;
   c.num_sms = num_sms;
@@ -307,11 +306,7 @@ int dpotrf_borrowed(int device, int num_sms, cudaStream_t st, int n, double* A, 
   c.graphs = false;
   c.allow_aux = false;  // one stream, no CUDA objects created on the caller's behalf
   c.d_status = d_status;
-  c.ws[1] = scratch;  // grow-only workspace that never needs to grow
-  c.ws_bytes[1] = scratch_bytes;
-  const int r = dpotrf(c, n, A, lda, st);
-  c.ws[1] = nullptr;  // borrowed: nothing to free
-  return r;
+  return dpotrf(c, n, A, lda, st);
 }
 
 std::string gkey(const char* op, std::initializer_list<long long> v) {

@@ -9,8 +9,8 @@
 //   applied to every column of A, matching the reference's full-row
 //   rawSwapRows (fromCol = 0, LU.hs:324-325).
 // dpotrf — right-looking blocked Cholesky, kNB = 128: diagonal block in SMEM,
-//   L21 = A21 L11^-T (inverse block times the panel, on the tensor cores), then
-//   A22 -= L21 L21^T as a lower-triangle-only GEMM (SYRK tile skip).  Same
+//   L21 = A21 L11^-T by substitution, then A22 -= L21 L21^T as a
+//   lower-triangle-only GEMM (SYRK tile skip).  Same
 //   mathematics as the reference's left-looking panelCholFactor
 //   (Chol.hs:279-321), different association.
 // dgetrs / dpotrs — blocked substitutions: a 128 x 128 triangular block
@@ -131,60 +131,29 @@ int dgetrf(Ctx& c, int n, double* A, long long lda, int* ipiv, cudaStream_t st) 
   return LM_OK;
 }
 
-namespace {
-
-// L21 = A21 inv(L11)^T for the block column at j0 (w wide, R rows below):
-// inv(L11) in one CTA, then the product with a copy of A21 on the DMMA GEMM.
-int potrf_panel(Ctx& c, double* A, long long lda, int j0, int w, int R, double* Linv, double* W21, cudaStream_t st,
-                int max_sms = 0) {
-  double* A11 = A + (long long)j0 * lda + j0;
-  double* A21 = A11 + (long long)w * lda;
-  {
-    Prof p(c, kPhaseTrsm, (double)w * w * w / 3.0, 16.0 * w * w, st);
-    LM_TRY(tri_inv_lower<double>(A11, lda, w, false, Linv, kNB, nullptr, st));
-  }
-  {
-    Prof p(c, kPhaseOther, 0.0, 16.0 * R * w, st);
-    LM_TRY(copy2d<double>(W21, kNB, A21, lda, R, w, st));
-  }
-  GemmDesc t;  // L21 = A21 * L11^-T
-  t.m = R; t.n = w; t.k = w; t.alpha = 1.0; t.beta = 0.0;
-  t.A = W21; t.lda = kNB; t.B = Linv; t.ldb = kNB; t.b_trans = true;
-  t.C = A21; t.ldc = lda;
-  t.max_sms = max_sms;
-  return dgemm(c, t, st);
-}
-
-}  // namespace
-
 // Right-looking blocked Cholesky with look-ahead: once the trailing update
 // has reached the next block column (its diagonal block and everything
 // below), that column is factored on the priority stream (diagonal block,
-// inverse, L21) while the rest of the lower-triangle update runs on the
+// L21) while the rest of the lower-triangle update runs on the
 // other SMs.  The two streams touch disjoint columns: the update reads the
 // current L21 and writes columns right of the next block column.
 int dpotrf(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
-  const size_t blk = (size_t)kNB * kNB;
-  void* ws = nullptr;
-  LM_TRY(ctx_workspace(c, 1, sizeof(double) * (blk + (size_t)n * kNB), &ws));
-  double* Linv = static_cast<double*>(ws);
-  double* W21 = Linv + blk;
   const int nsm = ctx_num_sms(c);
   const bool la = n >= kLookaheadMinN && nsm > 2 * kLookaheadSms && ctx_lookahead(c);
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   if (la) LM_TRY(ctx_aux(c, &aux, &ev_fork, &ev_join));
-  auto factor_column = [&](int j0, cudaStream_t s, int max_sms) {
+  auto factor_column = [&](int j0, cudaStream_t s) {
     const int w = std::min(kNB, n - j0);
     const int R = n - j0 - w;
     {
       Prof p(c, kPhasePanel, (double)w * w * w / 3.0, 8.0 * w * w, s);
-      LM_TRY(potrf_block<double>(c, A + (long long)j0 * lda + j0, lda, w, j0, s));
+      LM_TRY(potrf_block(c, A + (long long)j0 * lda + j0, lda, w, j0, s));
     }
-    if (R > 0) LM_TRY(potrf_panel(c, A, lda, j0, w, R, Linv, W21, s, max_sms));
-    return LM_OK;
+    Prof p(c, kPhaseTrsm, (double)R * w * w, 16.0 * R * w, s);
+    return chol_rows(c, A + (long long)j0 * lda + j0, lda, R, s);
   };
-  LM_TRY(factor_column(0, st, 0));
+  LM_TRY(factor_column(0, st));
   for (int j0 = 0; j0 < n; j0 += kNB) {
     const int w = std::min(kNB, n - j0);
     const int R = n - j0 - w;
@@ -207,7 +176,7 @@ int dpotrf(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
     if (la) {
       LM_CUDA_TRY(cudaEventRecord(ev_fork, st));
       LM_CUDA_TRY(cudaStreamWaitEvent(aux, ev_fork, 0));
-      LM_TRY(factor_column(j0 + w, aux, kLookaheadSms));
+      LM_TRY(factor_column(j0 + w, aux));
       LM_CUDA_TRY(cudaEventRecord(ev_join, aux));
       if (rest > 0) {
         r.max_sms = nsm - kLookaheadSms;
@@ -216,7 +185,7 @@ int dpotrf(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
       LM_CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
     } else {
       if (rest > 0) LM_TRY(dgemm(c, r, st));
-      LM_TRY(factor_column(j0 + w, st, 0));
+      LM_TRY(factor_column(j0 + w, st));
     }
   }
   return zero_upper<double>(A, lda, n, st);

@@ -203,8 +203,10 @@ int panel_ctas(Ctx& c, int rows);
 
 // Cholesky of a w x w diagonal block (w <= 128) in place, lower triangle;
 // records the first non-positive pivot (global index base + j + 1) in status[1].
-template <typename T>
-int potrf_block(Ctx& c, T* A, long long lda, int w, int base, cudaStream_t st);
+int potrf_block(Ctx& c, double* A, long long lda, int w, int base, cudaStream_t st);
+// The R rows below a factored 128 x 128 diagonal block A11, same columns:
+// A21 <- A21 L11^-T.
+int chol_rows(Ctx& c, double* A11, long long lda, int R, cudaStream_t st);
 
 // Mixed precision (ir.cu): FP32 LU with TF32 tensor-core updates, FP32
 // substitutions, FP64 refinement.  `factor_runner` runs the factorisation
@@ -233,10 +235,9 @@ int rbt_transform(float* Ar, long long ldr, const double* A, long long lda, int 
                   const double* dv, cudaStream_t st);
 int rbt_rows(float* D, long long ldd, int np, int nrhs, const double* d, bool transposed, cudaStream_t st);
 
-// Run dpotrf with caller-provided device scratch (workspace slot 1) and
-// status words instead of a context's own allocations (api.cu).
-int dpotrf_borrowed(int device, int num_sms, cudaStream_t st, int n, double* A, long long lda, int* d_status,
-                    void* scratch, size_t scratch_bytes);
+// Run dpotrf (which needs no scratch) with the caller's status words instead of
+// a context's own (api.cu).
+int dpotrf_borrowed(int device, int num_sms, cudaStream_t st, int n, double* A, long long lda, int* d_status);
 
 // r = b - A x for nrhs columns (FP64), and max-norm helpers (resid.cu).
 int dresidual(Ctx& c, int n, int nrhs, const double* A, long long lda, const double* X, long long ldx,

@@ -1,4 +1,4 @@
-// Panel kernels: the latency-bound, column-by-column parts of LU and Cholesky.
+// Panel kernel: the latency-bound, column-by-column part of LU.
 //
 // panel_lu  — partial-pivoting LU of a whole panel (rows [c0, n), up to 128
 //   columns) in one launch, the B200 replacement for panelLUFactor's column
@@ -30,10 +30,6 @@
 //   and interchanges between the four of them (8192 rows).
 //   NaN rule of the reference scan: if |a_jj| is NaN it stays the pivot; NaNs
 //   below it never win.
-//
-// potrf_block — Cholesky of one <=128 x 128 diagonal block in shared memory,
-//   by 32-column panels (rawCholColumnSIMDFrom, K.hs:2137-2195, for a
-//   diagonal panel).
 #include <algorithm>
 #include <climits>
 
@@ -815,178 +811,5 @@ template int panel_ctas<double>(Ctx&, int);
 template int panel_ctas<float>(Ctx&, int);
 template int panel_lu<double>(Ctx&, double*, long long, int, int, int, int*, int*, cudaStream_t);
 template int panel_lu<float>(Ctx&, float*, long long, int, int, int, int*, int*, cudaStream_t);
-
-// ---------------------------------------------------------------------------
-// Cholesky of one diagonal block (w <= 128), by 32-column panels in shared memory.
-// ---------------------------------------------------------------------------
-namespace {
-
-// Cholesky of the w x w block at A (w <= 128, lower triangle) in place, in
-// shared memory, right-looking by 32-column panels (padded to whole panels
-// with the identity).  Per panel c0:
-//   1. warp 0 factors the 32 x 32 diagonal block in registers: lane i holds
-//      row i; step k broadcasts a_kk, forms r = 1 / sqrt(a_kk), l_ik = a_ik r
-//      (l_kk = a_kk r) and subtracts l_ik l_jk from the lanes' later columns
-//      with one shuffle per column (steps unrolled at compile time so the row
-//      stays in registers: 256 threads leave room for it); r is kept for the
-//      panel solve;
-//   2. one thread per row below solves x = a L11^-T by the same products
-//      (x_k = (a_k - sum_{j<k} x_j l_kj) r_k);
-//   3. all threads subtract X X^T from the lower trailing block in 4 x 4
-//      register tiles.
-// A non-positive (or NaN) pivot is recorded as base + k + 1 in status[1]
-// (the first one: panels and steps run in order); the arithmetic continues,
-// leaving the NaN the reference's would.
-constexpr int kPbLd = 129;  // padded row stride of the shared copy (elements)
-constexpr int kPbXt = 96;   // row stride of the transposed panel X^T (elements)
-constexpr int kPbThreads = 256;
-
-template <typename T>
-constexpr int potrf_block_smem() {
-  return (128 * kPbLd + 32 * kPbXt) * (int)sizeof(T);
-}
-
-// Step K of the one-warp 32 x 32 Cholesky (lane i holds row i in d), with
-// K a compile-time constant so that d stays in registers.
-template <typename T, int K>
-__device__ __forceinline__ void pb_diag_step(T (&d)[32], int lane, int& bad, T& myr) {
-  if constexpr (K < 32) {
-    const T dkk = __shfl_sync(0xffffffffu, d[K], K);
-    bad = (bad < 0 && !(dkk > T(0))) ? K : bad;  // the same in every lane
-    const T r = rsqrt(dkk);
-    const T lk = d[K] * r;
-    d[K] = lane >= K ? lk : d[K];
-    myr = lane == K ? r : myr;
-#pragma unroll
-    for (int j = K + 1; j < 32; ++j) {
-      const T lj = __shfl_sync(0xffffffffu, lk, j);
-      d[j] = lane >= j ? fma(-lk, lj, d[j]) : d[j];
-    }
-    pb_diag_step<T, K + 1>(d, lane, bad, myr);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) potrf_block_kernel(T* A, long long lda, int w, int base, int* status) {
-  extern __shared__ __align__(16) unsigned char pb_smem[];
-  T* S = reinterpret_cast<T*>(pb_smem);  // 128 x kPbLd, lower triangle
-  T* Xt = S + 128 * kPbLd;               // 32 x kPbXt: the solved panel, transposed
-  __shared__ T rdiag[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int np = (w + 31) >> 5;  // panels
-  const int wp = np << 5;        // padded order
-  for (int e = tid; e < wp * wp; e += kPbThreads) {
-    const int i = e / wp, j = e % wp;
-    T v = T(0);
-    if (j <= i) v = (i < w) ? A[(long long)i * lda + j] : (i == j ? T(1) : T(0));
-    S[i * kPbLd + j] = v;
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int p = 0; p < np; ++p) {
-    const int c0 = p << 5;
-    // ---- 1. diagonal block, one warp (selects, not branches: the warp
-    //         stays converged for its shuffles) ----
-    if (warp == 0) {
-      T d[32];
-      T* row = S + (c0 + lane) * kPbLd + c0;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) d[j] = row[j];
-      int bad = -1;
-      T myr = T(0);
-      pb_diag_step<T, 0>(d, lane, bad, myr);
-      rdiag[lane] = myr;
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j <= lane) row[j] = d[j];
-      if (lane == 0 && bad >= 0 && c0 + bad < w) atomicCAS(status + 1, 0, base + c0 + bad + 1);
-    }
-    __syncthreads();
-    const int m = wp - c0 - 32;  // rows below the diagonal block
-    if (m <= 0) break;
-    // ---- 2. panel solve, one thread per row: x = a L11^-T ----
-    if (tid < m) {
-      T* row = S + (c0 + 32 + tid) * kPbLd + c0;
-      const T* L = S + c0 * kPbLd + c0;
-      T a[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) a[j] = row[j];
-#pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        const T x = a[k] * rdiag[k];
-        a[k] = x;
-#pragma unroll
-        for (int j = k + 1; j < 32; ++j) a[j] = fma(-x, L[j * kPbLd + k], a[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        row[j] = a[j];
-        Xt[j * kPbXt + tid] = a[j];
-      }
-    }
-    __syncthreads();
-    // ---- 3. trailing update, 4 x 4 register tiles of the lower triangle ----
-    const int tt = m >> 2;                 // tiles per side
-    const int ntiles = tt * (tt + 1) / 2;  // tile (ti, tj), tj <= ti, at t = ti (ti + 1) / 2 + tj
-    for (int t = tid; t < ntiles; t += kPbThreads) {
-      int ti = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-      while (ti > 0 && ti * (ti + 1) / 2 > t) --ti;
-      while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-      const int tj = t - ti * (ti + 1) / 2;
-      const int ri = 4 * ti, rj = 4 * tj;  // rows within the trailing block
-      const int i0 = c0 + 32 + ri, j0 = c0 + 32 + rj;
-      T acc[4][4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = S[(i0 + u) * kPbLd + j0 + v];
-#pragma unroll 8
-      for (int k = 0; k < 32; ++k) {
-        T xi[4], xj[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          xi[u] = Xt[k * kPbXt + ri + u];
-          xj[u] = Xt[k * kPbXt + rj + u];
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u][v] = fma(-xi[u], xj[v], acc[u][v]);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (j0 + v <= i0 + u) S[(i0 + u) * kPbLd + j0 + v] = acc[u][v];
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < w * w; e += kPbThreads) {
-    const int i = e / w, j = e % w;
-    if (j <= i) A[(long long)i * lda + j] = S[i * kPbLd + j];
-  }
-}
-
-}  // namespace
-
-template <typename T>
-int potrf_block(Ctx& c, T* A, long long lda, int w, int base, cudaStream_t st) {
-  if (w <= 0) return LM_OK;
-  if (w > 128) return LM_ERR_ARG;
-  constexpr int smem = potrf_block_smem<T>();
-  static bool attr_set[kMaxDevices] = {};
-  const int dev = ctx_device(c);
-  if (!attr_set[dev]) {
-    LM_CUDA_TRY(cudaFuncSetAttribute(potrf_block_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr_set[dev] = true;
-  }
-  potrf_block_kernel<T><<<1, kPbThreads, smem, st>>>(A, lda, w, base, ctx_status(c));
-  count_launch(1);
-  LM_CUDA_TRY(cudaGetLastError());
-  return LM_OK;
-}
-
-template int potrf_block<double>(Ctx&, double*, long long, int, int, cudaStream_t);
-template int potrf_block<float>(Ctx&, float*, long long, int, int, cudaStream_t);
 
 }  // namespace lm
