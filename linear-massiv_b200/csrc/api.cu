@@ -47,7 +47,7 @@ struct Ctx {
   int num_sms = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  int* d_status = nullptr;  // int[4], see common.cuh
+  int* d_status = nullptr;  // int[8], see ctx_status
   void* ws[kWsSlots] = {};
   size_t ws_bytes[kWsSlots] = {};
   std::mutex mu;
@@ -374,13 +374,13 @@ int lm_ctx_create(lm_ctx** out, int device) {
   ctx->c.device = device;
   ctx->c.num_sms = prop.multiProcessorCount;
   if (cudaStreamCreateWithFlags(&ctx->c.stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&ctx->c.d_status, 4 * sizeof(int)) != cudaSuccess) {
+      cudaMalloc(&ctx->c.d_status, 8 * sizeof(int)) != cudaSuccess) {
     lm::set_last_error("context allocation failed");
     delete ctx;
     return LM_ERR_CUDA;
   }
   ctx->c.own_stream = true;
-  cudaMemset(ctx->c.d_status, 0, 4 * sizeof(int));
+  cudaMemset(ctx->c.d_status, 0, 8 * sizeof(int));
   *out = ctx;
   return LM_OK;
 }

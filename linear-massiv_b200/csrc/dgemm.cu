@@ -3,20 +3,31 @@
 // Replaces linear-massiv's rawGemmKernel family (Internal/Kernel.hs:145-806:
 // the 4x8 AVX2 register-blocked micro-kernel over 64^3 cache blocks, with
 // B-panel packing above min dimension 96).  On B200 the "cache blocking" is a
-// 128 x 128 (or 128 x 64) CTA tile, the "packing" is a TMA tile load into
-// 128-byte-swizzled shared memory, and the "micro-kernel" is a warp tile of
-// 64 x 32 FP64 accumulators fed by DMMA.
+// 64 x 64 CTA tile, the "packing" is a TMA tile load into 128-byte-swizzled
+// shared memory, and the "micro-kernel" is a warp tile of 32 x 32 FP64
+// accumulators fed by DMMA.
 //
-// Structure (one CTA per SM, persistent over output tiles):
+// Structure (two or three CTAs per SM, persistent over output tiles):
 //   warp NC       : TMA producer (one elected lane) filling a STAGES-deep ring
 //                   of A/B k-slices (16 doubles = 128 B deep), mbarrier-tracked;
-//   warps 0..NC-1 : consumers, each a 64 x 32 warp tile of m16n8k4 DMMAs,
+//   warps 0..NC-1 : consumers, each a 32 x 32 warp tile of m16n8k4 DMMAs,
 //                   then a fused epilogue C = alpha*acc + beta*C (in place),
 //                   optionally restricted to the lower triangle (SYRK tiles).
 // Short-k updates with beta != 0 (the factorisations' trailing updates) stage
 // each C tile in shared memory: the producer TMA-loads it while the tile's
 // main loop runs, so the epilogue reads C on chip instead of waiting on
-// L2/HBM (at k = 128 those waits were about a third of the time).
+// L2/HBM.  The CTAs of an SM drift apart, so that one's epilogue and first loads
+// run under the others' DMMAs, and small tiles leave less of the last wave idle.
+// Against 128 x 128 tiles with one CTA per SM (before):
+//   k = 128, beta = 1 : m = n = 8192 591 -> 579 us, 16384 2316 -> 2271 us,
+//                       8192 x 128 24.9 -> 15.5 us, 8192 x 64 22.8 -> 11.5 us;
+//   square            : 500 80 -> 27 us, 1000 150 -> 76 us, 2000 (1500 x 1002)
+//                       289 -> 226 us, 4096 4.05 -> 3.94 ms, 8192 32.1 -> 31.2 ms.
+// Tiles go to CTAs by index, or, for a product that runs beside other kernels (the
+// trailing updates beside a panel), by tickets: CTAs that find their SM taken start
+// when it is free and take what is left, and SMs can be kept clear for a kernel
+// still to come.  A ticket travels from the producer to the consumers with the first
+// k-slice of its tile.
 // No cluster multicast is used anywhere.
 #include "common.cuh"
 #include "internal.h"
@@ -44,8 +55,11 @@ struct GemmArgs {
   double* C;
   long long ldc;
   int lower_only;
+  uint32_t zero;   // 0
   int prefetch_c;  // TMA-prefetch each C tile into L2 when its main loop starts
   int tiles_m, tiles_n, num_tiles;
+  int* sched;    // tickets: next tile, CTAs done, CTAs sent away (zero between launches), or null: tiles by CTA index
+  int smid_end;  // with tickets, CTAs on SMs from here on are sent away (half of them at most)
   int* status;
 };
 
@@ -56,26 +70,11 @@ __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* tmap, int 
                : "memory");
 }
 
-// MINB CTAs share an SM: with two, one CTA's epilogue (C read-modify-write)
-// overlaps the other's DMMA main loop, which matters for the short-k
-// trailing updates of the factorisations.
-template <int BM, int BN, int MINB, bool CSM = false>
+// MINB CTAs share an SM.
+template <int BM, int BN, int WM, int MINB, bool CSM = false>
 struct GemmCfg {
-  static constexpr int NC = (BM / 64) * (BN / 32);  // consumer warps
-  // Short-k update (CSM): the producer is a whole warpgroup so that
-  // setmaxnreg can move its registers to the consumers (a lone producer warp
-  // puts three warps on one SM sub-partition, which caps every thread at 168
-  // registers and spills the 64 x 32 FP64 accumulator tile in the main loop;
-  // at k = 128 that cost 17%, while the long-k kernel measured the same
-  // either way)
-  static constexpr bool SPLIT_REGS = CSM && NC == 8 && MINB == 1;
-  static constexpr int PRODUCER_WARPS = SPLIT_REGS ? 4 : 1;
-  static constexpr int THREADS = (NC + PRODUCER_WARPS) * 32;
-  static constexpr int LAUNCH_REGS = 168;  // 65536 / 384, rounded down to 8
-  static constexpr int CONSUMER_REGS = 232, PRODUCER_REGS = 40;
-  static_assert(!SPLIT_REGS || NC * 32 * CONSUMER_REGS + PRODUCER_WARPS * 32 * PRODUCER_REGS <=
-                                     THREADS * LAUNCH_REGS,
-                "register split must fit in what the CTA is launched with");
+  static constexpr int NC = (BM / WM) * (BN / 32);  // consumer warps, WM x 32 each
+  static constexpr int THREADS = (NC + 1) * 32;  // one producer warp
   static constexpr int A_BYTES = BM * kBK * 8;
   static constexpr int B_BYTES = BN * kBK * 8;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -83,7 +82,7 @@ struct GemmCfg {
   static constexpr int C_BYTES = CSM ? BM * BN * 8 : 0;
   static constexpr int BUDGET = CSM ? (227 * 1024 - 2048) / MINB - C_BYTES : (200 * 1024) / MINB;
   static constexpr int STAGES = BUDGET / STAGE_BYTES > 8 ? 8 : BUDGET / STAGE_BYTES;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + C_BYTES + 2 * STAGES * 8 + 16 + 1024;  // + alignment slack
+  static constexpr int SMEM = STAGES * STAGE_BYTES + C_BYTES + STAGES * (2 * 8 + 4) + 16 + 1024;  // + alignment slack
   static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
   static_assert(STAGES >= 2, "operand ring depth");
 };
@@ -110,12 +109,13 @@ __device__ __forceinline__ void tile_coords(const GemmArgs& g, int t, int& tm, i
 
 // CSM: C staged in shared memory (tmC then maps 16-double x BM boxes with the
 // 128-byte swizzle); requires beta != 0.
-template <int BM, int BN, bool AT, bool BT, int MINB, bool CSM>
-__global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
+template <int BM, int BN, int WM, bool AT, bool BT, int MINB, bool CSM>
+__global__ void __launch_bounds__(GemmCfg<BM, BN, WM, MINB, CSM>::THREADS, MINB)
     dgemm_dmma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmC, GemmArgs g) {
-  using Cfg = GemmCfg<BM, BN, MINB, CSM>;
+  using Cfg = GemmCfg<BM, BN, WM, MINB, CSM>;
   constexpr int STAGES = Cfg::STAGES;
+  constexpr int MI = WM / 16;  // MMA rows of a warp tile
   constexpr int C_BOX = BM * 16 * 8;  // bytes of one staged C box
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -127,10 +127,37 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
   uint64_t* empty = full + STAGES;
   uint64_t* cfull = empty + STAGES;  // C tile landed
   uint64_t* cempty = cfull + 1;      // every consumer warp has read it
+  int* tile_of = reinterpret_cast<int*>(cempty + 1);  // tile that starts in a ring slot, or -1: no more
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int KT = (g.k + kBK - 1) / kBK;
+  // thread 0 of the producer warp leaves last; the last CTA clears the tickets
+  auto leave = [&]() {
+    if (g.sched) {
+      __threadfence();
+      if (atomicAdd(g.sched + 1, 1) == (int)gridDim.x - 1) {
+        g.sched[0] = 0;
+        g.sched[1] = 0;
+        g.sched[2] = 0;
+      }
+    }
+  };
+  if (g.sched) {
+    uint32_t smid;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+    if ((int)smid >= g.smid_end) {  // uniform over the CTA
+      // whichever SMs the CTAs land on, half of them stay and take every tile
+      if (threadIdx.x == 0) *tile_of = atomicAdd(g.sched + 2, 1) < (int)gridDim.x / 2;
+      __syncthreads();
+      const bool away = *tile_of != 0;
+      __syncthreads();
+      if (away) {
+        if (threadIdx.x == 0) leave();
+        return;
+      }
+    }
+  }
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -145,21 +172,23 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
 
   if (warp >= Cfg::NC) {
     // ---------------- producer ----------------
-    if constexpr (Cfg::SPLIT_REGS)
-      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::PRODUCER_REGS) : "memory");
     if (warp == Cfg::NC && lane == 0) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       if (CSM) tma_prefetch_desc(&tmC);
       int it = 0, cj = 0;
-      for (int t = blockIdx.x; t < g.num_tiles; t += gridDim.x, ++cj) {
+      int t = g.sched ? atomicAdd(g.sched, 1) : (int)blockIdx.x;
+      for (; t < g.num_tiles; ++cj) {
         int tm, tn;
         tile_coords(g, t, tm, tn);
+        const int tile = t;
+        t = g.sched ? atomicAdd(g.sched, 1) : t + (int)gridDim.x;
         if (!CSM && g.prefetch_c) tma_prefetch_l2_2d(&tmC, tn * BN, tm * BM);
         for (int kb = 0; kb < KT; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (uint32_t)((it / STAGES) & 1) ^ 1u;
-          if (!mbar_wait(&empty[s], ph, g.status)) return;
+          if (!mbar_wait(&empty[s], ph, g.status)) return leave();
+          if (kb == 0) tile_of[s] = tile;
           mbar_arrive_expect_tx(&full[s], Cfg::STAGE_BYTES);
           if (AT) {
 #pragma unroll
@@ -179,20 +208,24 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
             // this tile's C, once the previous tile's epilogue has read the
             // buffer; issued after the first ring slots so that the main
             // loop never waits on it
-            if (!mbar_wait(cempty, (uint32_t)(cj & 1) ^ 1u, g.status)) return;
+            if (!mbar_wait(cempty, (uint32_t)(cj & 1) ^ 1u, g.status)) return leave();
             mbar_arrive_expect_tx(cfull, Cfg::C_BYTES);
 #pragma unroll
             for (int j = 0; j < BN / 16; ++j) tma_load_2d(sC + j * C_BOX, &tmC, tn * BN + j * 16, tm * BM, cfull);
           }
         }
       }
+      const int s = it % STAGES;  // tell the consumers
+      if (mbar_wait(&empty[s], (uint32_t)((it / STAGES) & 1) ^ 1u, g.status)) {
+        tile_of[s] = -1;
+        mbar_arrive(&full[s]);
+      }
+      leave();
     }
     return;
   }
 
   // ---------------- consumers ----------------
-  if constexpr (Cfg::SPLIT_REGS)
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::CONSUMER_REGS) : "memory");
   const int wm = warp / (BN / 32);
   const int wn = warp % (BN / 32);
   const int gq = lane >> 2;  // groupID
@@ -200,13 +233,16 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
   const uint32_t sA32 = smem_u32(sA);
   const uint32_t sB32 = smem_u32(sB);
 
-  int it = 0, cj = 0;
-  for (int t = blockIdx.x; t < g.num_tiles; t += gridDim.x, ++cj) {
+  int it = 0;
+  for (int cj = 0;; ++cj) {
+    if (!mbar_wait(&full[it % STAGES], (uint32_t)((it / STAGES) & 1), g.status)) return;
+    const int t = tile_of[it % STAGES];
+    if (t < 0) break;
     int tm, tn;
     tile_coords(g, t, tm, tn);
-    double acc[4][4][4];
+    double acc[MI][4][4];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < MI; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b)
 #pragma unroll
@@ -221,13 +257,14 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
       __syncwarp();
       const uint32_t aBase = sA32 + s * Cfg::A_BYTES;
       const uint32_t bBase = sB32 + s * Cfg::B_BYTES;
+      uint32_t read = 0;  // depends on the last operands read from the slot
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
-        double af[4][2], bf[4];
+        double af[MI][2], bf[4];
         const int kc = kk * 4 + tq;
 #pragma unroll
-        for (int mi = 0; mi < 4; ++mi) {
-          const int r = wm * 64 + mi * 16 + gq;
+        for (int mi = 0; mi < MI; ++mi) {
+          const int r = wm * WM + mi * 16 + gq;
           if (AT) {
             af[mi][0] = lds_f64(aBase + (r >> 4) * 2048 + swz128(kc, r & 15));
             af[mi][1] = lds_f64(aBase + ((r + 8) >> 4) * 2048 + swz128(kc, (r + 8) & 15));
@@ -245,12 +282,23 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
             bf[ni] = lds_f64(bBase + (nl >> 4) * 2048 + swz128(kc, nl & 15));
         }
 #pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
+        for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
           for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
+        if (kk == 3) {
+#pragma unroll
+          for (int mi = 0; mi < MI; ++mi) read |= __double2hiint(af[mi][0]) | __double2hiint(af[mi][1]);
+#pragma unroll
+          for (int ni = 0; ni < 4; ++ni) read |= __double2hiint(bf[ni]);
+        }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
+      // The slot is given back only when its operands are in registers: an arrive
+      // that merely follows the loads in program order was seen to overtake them
+      // when other warps' epilogues filled the memory pipe (their products can be
+      // scheduled after it), and the next tile's TMA then overwrote them.  g.zero
+      // is 0, which the compiler does not know.
+      if (lane == 0) mbar_arrive(&empty[s] + (read & g.zero));
     }
 
     // ---------------- epilogue: C = alpha*acc + beta*C ----------------
@@ -262,10 +310,10 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
       __syncwarp();
       const uint32_t sC32 = smem_u32(sC);
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
+      for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int rl = wm * 64 + mi * 16 + gq + h * 8;  // row within the tile
+          const int rl = wm * WM + mi * 16 + gq + h * 8;  // row within the tile
           const int row = tm * BM + rl;
 #pragma unroll
           for (int ni = 0; ni < 4; ++ni) {
@@ -293,11 +341,11 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
       if (lane == 0) mbar_arrive(cempty);
     } else {
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi) {
+      for (int mi = 0; mi < MI; ++mi) {
         double old[2][4][2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int row = tm * BM + wm * 64 + mi * 16 + gq + h * 8;
+          const int row = tm * BM + wm * WM + mi * 16 + gq + h * 8;
           const double* crow = g.C + (long long)row * g.ldc;
 #pragma unroll
           for (int ni = 0; ni < 4; ++ni) {
@@ -320,7 +368,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, MINB, CSM>::THREADS, MINB)
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int row = tm * BM + wm * 64 + mi * 16 + gq + h * 8;
+          const int row = tm * BM + wm * WM + mi * 16 + gq + h * 8;
           if (row >= g.m) continue;
           double* crow = g.C + (long long)row * g.ldc;
 #pragma unroll
@@ -354,22 +402,14 @@ __global__ void scale_kernel(double* C, long long ldc, int m, int n, double beta
   }
 }
 
-template <int BM, int BN, bool AT, bool BT, int MINB, bool CSM = false>
+template <int BM, int BN, int WM, bool AT, bool BT, int MINB, bool CSM = false>
 int launch_dmma(Ctx& ctx, const GemmDesc& d, cudaStream_t st) {
-  using Cfg = GemmCfg<BM, BN, MINB, CSM>;
+  using Cfg = GemmCfg<BM, BN, WM, MINB, CSM>;
   static bool attr_set[kMaxDevices] = {};  // per instantiation and device, set under the API lock
-  auto kern = dgemm_dmma_kernel<BM, BN, AT, BT, MINB, CSM>;
+  auto kern = dgemm_dmma_kernel<BM, BN, WM, AT, BT, MINB, CSM>;
   const int dev = ctx_device(ctx);
   if (!attr_set[dev]) {
     LM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
-    if (Cfg::SPLIT_REGS) {
-      // the setmaxnreg split assumes the CTA is launched with LAUNCH_REGS per
-      // thread; with fewer the consumers' increase could never be granted,
-      // so the caller falls back to another kernel
-      cudaFuncAttributes fa;
-      LM_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
-      if (fa.numRegs < Cfg::LAUNCH_REGS) return LM_ERR_UNSUPPORTED;
-    }
     attr_set[dev] = true;
   }
   CUtensorMap tmA, tmB;
@@ -397,6 +437,7 @@ int launch_dmma(Ctx& ctx, const GemmDesc& d, cudaStream_t st) {
   else
     tmC = tmA;  // unused
   GemmArgs g;
+  g.zero = 0;
   g.prefetch_c = c_ok ? 1 : 0;
   g.m = d.m; g.n = d.n; g.k = d.k;
   g.alpha = d.alpha; g.beta = d.beta;
@@ -406,8 +447,11 @@ int launch_dmma(Ctx& ctx, const GemmDesc& d, cudaStream_t st) {
   g.tiles_n = cdiv(d.n, BN);
   g.num_tiles = d.lower_only ? g.tiles_m * (g.tiles_m + 1) / 2 : g.tiles_m * g.tiles_n;
   g.status = ctx_status(ctx);
-  const int sms = d.max_sms > 0 ? std::min(d.max_sms, ctx_num_sms(ctx)) : ctx_num_sms(ctx);
-  int grid = std::min(g.num_tiles, MINB * sms);
+  const int sms = ctx_num_sms(ctx);
+  const int grid = std::min(g.num_tiles, MINB * sms);
+  // tickets only where more tiles than CTAs are left to give out, or SMs to keep clear
+  g.sched = d.sched && (g.num_tiles > grid || d.keep_sms > 0) ? d.sched : nullptr;
+  g.smid_end = sms - d.keep_sms;
   kern<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(tmA, tmB, tmC, g);
   count_launch(1);
   LM_CUDA_TRY(cudaGetLastError());
@@ -434,44 +478,24 @@ int dgemm(Ctx& ctx, const GemmDesc& d, cudaStream_t st) {
       (d.lda & 1) || (d.ldb & 1))
     return LM_ERR_UNSUPPORTED;
   if (d.a_trans && d.b_trans) return LM_ERR_UNSUPPORTED;
-  // Short k with beta != 0 (the factorisations' trailing updates): 128 x 128
-  // tiles with C staged in shared memory.  Other short-k or narrow products:
-  // 128 x 64 tiles, two CTAs per SM.  Long k: 128 x 128 tiles, one CTA per
-  // SM, deeper pipeline.
+  // Short k with beta != 0 (the factorisations' trailing updates): C staged in
+  // shared memory, three CTAs per SM with two k-slices each in flight.  Beyond
+  // k = 256 the C traffic no longer counts and a deeper ring does: two CTAs per SM
+  // (4096^3: 3.97 ms, and 4.18 ms with three; k = 128, m = n = 4000: 0.195 ms with
+  // two and 0.147 ms with three).
   const double flops = d.lower_only ? (double)d.m * (d.m + 1) * d.k : 2.0 * d.m * d.n * d.k;
   const double bytes = 8.0 * ((double)d.m * d.k + (double)d.k * d.n +
                               (d.beta != 0.0 ? 2.0 : 1.0) * (d.lower_only ? 0.5 : 1.0) * d.m * d.n);
   Prof prof(ctx, kPhaseGemm, flops, bytes, st);
-  const bool narrow = (d.n <= 64 || d.k <= 256) && !d.lower_only;
   const bool c_tma = d.beta != 0.0 && !(reinterpret_cast<uintptr_t>(d.C) & 15) && !(d.ldc & 1);
-  const int sms = d.max_sms > 0 ? std::min(d.max_sms, ctx_num_sms(ctx)) : ctx_num_sms(ctx);
-  if (d.k <= 256 && d.n > 64 && c_tma && !d.lower_only && cdiv(d.m, 128) * cdiv(d.n, 128) < sms) {
-    // not one 128 x 128 tile per SM (a panel's own columns, the end of a
-    // factorisation): a quarter of the tile in about half the time
-    if (d.a_trans) return launch_dmma<64, 64, true, false, 2, true>(ctx, d, st);
-    if (d.b_trans) return launch_dmma<64, 64, false, true, 2, true>(ctx, d, st);
-    return launch_dmma<64, 64, false, false, 2, true>(ctx, d, st);
+  if (d.k <= 256 && c_tma) {
+    if (d.a_trans) return launch_dmma<64, 64, 32, true, false, 3, true>(ctx, d, st);
+    if (d.b_trans) return launch_dmma<64, 64, 32, false, true, 3, true>(ctx, d, st);
+    return launch_dmma<64, 64, 32, false, false, 3, true>(ctx, d, st);
   }
-  if (d.k <= 256 && d.n > 64 && c_tma) {
-    int rc;
-    if (d.a_trans)
-      rc = launch_dmma<128, 128, true, false, 1, true>(ctx, d, st);
-    else if (d.b_trans)
-      rc = launch_dmma<128, 128, false, true, 1, true>(ctx, d, st);
-    else
-      rc = launch_dmma<128, 128, false, false, 1, true>(ctx, d, st);
-    // LM_ERR_UNSUPPORTED before any launch: compiled with fewer registers
-    // than the register split needs; the kernels below take the update
-    if (rc != LM_ERR_UNSUPPORTED) return rc;
-  }
-  if (d.a_trans)
-    return narrow ? launch_dmma<128, 64, true, false, 2>(ctx, d, st)
-                  : launch_dmma<128, 128, true, false, 1>(ctx, d, st);
-  if (d.b_trans)
-    return narrow ? launch_dmma<128, 64, false, true, 2>(ctx, d, st)
-                  : launch_dmma<128, 128, false, true, 1>(ctx, d, st);
-  return narrow ? launch_dmma<128, 64, false, false, 2>(ctx, d, st)
-                : launch_dmma<128, 128, false, false, 1>(ctx, d, st);
+  if (d.a_trans) return launch_dmma<64, 64, 32, true, false, 2>(ctx, d, st);
+  if (d.b_trans) return launch_dmma<64, 64, 32, false, true, 2>(ctx, d, st);
+  return launch_dmma<64, 64, 32, false, false, 2>(ctx, d, st);
 }
 
 }  // namespace lm

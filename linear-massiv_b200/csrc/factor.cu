@@ -28,29 +28,28 @@ namespace {
 
 constexpr int kNB = 128;
 
-
 // B (w x ncols, ldb) <- inv(unit lower L11) B (the no-pivot factorisation's
 // row block).  Small blocks in one fused launch; otherwise inv(L11) (Linv,
-// kNB x kNB scratch) times B on the tensor cores, written in place: with
-// m = w <= 128 there is one row of output tiles, so each CTA reads exactly
-// the columns of B that it later overwrites, all of them before its epilogue,
-// and no other CTA reads them.
+// kNB x kNB scratch) times a copy of B (W, kNB x (ncols + 1) scratch) on the
+// tensor cores.
 int trsm_unit_lower_gemm(Ctx& c, const double* L11, long long lda, int w, double* B, long long ldb, int ncols,
-                         double* Linv, cudaStream_t st) {
+                         double* Linv, double* W, cudaStream_t st) {
   if (w <= 0 || ncols <= 0) return LM_OK;
   if (w <= 64 && ncols <= 128) {
     Prof p(c, kPhaseTrsm, (double)w * w * ncols, 8.0 * ((double)w * w / 2 + 2.0 * w * ncols), st);
     return trsm_lower_small<double>(L11, lda, w, true, B, ldb, ncols, st);
   }
+  const long long ldw = (ncols + 1) & ~1;
   {
-    Prof p(c, kPhaseTrsm, (double)w * w * w / 3.0, 8.0 * (double)w * w, st);
+    Prof p(c, kPhaseTrsm, (double)w * w * w / 3.0, 8.0 * (double)w * w + 16.0 * w * ncols, st);
     LM_TRY(tri_inv_lower<double>(L11, lda, w, true, Linv, kNB, nullptr, st));
+    LM_TRY(copy2d<double>(W, ldw, B, ldb, w, ncols, st));
   }
   GemmDesc d;
   d.m = w; d.n = ncols; d.k = w;
   d.alpha = 1.0; d.beta = 0.0;
   d.A = Linv; d.lda = kNB;
-  d.B = B; d.ldb = ldb;
+  d.B = W; d.ldb = ldw;
   d.C = B; d.ldc = ldb;
   return dgemm(c, d, st);
 }
@@ -66,7 +65,7 @@ constexpr int kLookaheadMinN = 384;
 // the interchanges, block solve and update of its own 128 columns.  With
 // look-ahead it is then factored on the priority stream while the same three
 // operations run on the rest of the matrix, on the SMs that the panel's
-// cluster leaves.  Nothing waits across the two streams inside a kernel; at
+// cluster leaves and, once it is done, on those too (tiles by ticket).  Nothing waits across the two streams inside a kernel; at
 // worst the panel starts when the update ends.
 int dgetrf(Ctx& c, int n, double* A, long long lda, int* ipiv, cudaStream_t st) {
   int* plan[2];  // row plans of the current panel and of the one factored beside its update
@@ -119,7 +118,7 @@ int dgetrf(Ctx& c, int n, double* A, long long lda, int* ipiv, cudaStream_t st) 
       LM_CUDA_TRY(cudaStreamWaitEvent(aux, ev_fork, 0));
       LM_TRY(panel(nx, aux));
       LM_CUDA_TRY(cudaEventRecord(ev_join, aux));
-      r.max_sms = nsm - panel_ctas<double>(c, m);
+      r.sched = ctx_status(c) + 2;
     }
     LM_TRY(rows(0, k0, rx, n));
     if (r.n > 0) LM_TRY(dgemm(c, r, st));
@@ -179,7 +178,8 @@ int dpotrf(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
       LM_TRY(factor_column(j0 + w, aux));
       LM_CUDA_TRY(cudaEventRecord(ev_join, aux));
       if (rest > 0) {
-        r.max_sms = nsm - kLookaheadSms;
+        r.sched = ctx_status(c) + 2;
+        r.keep_sms = kLookaheadSms;
         LM_TRY(dgemm(c, r, st));
       }
       LM_CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
@@ -217,7 +217,7 @@ int dgetrf_nopiv(Ctx& c, int n, double* A, long long lda, cudaStream_t st) {
     if (R <= 0) break;
     double* A12 = A11 + w;
     double* A21 = A11 + (long long)w * lda;
-    LM_TRY(trsm_unit_lower_gemm(c, A11, lda, w, A12, lda, R, Linv, st));
+    LM_TRY(trsm_unit_lower_gemm(c, A11, lda, w, A12, lda, R, Linv, W21, st));
     {
       Prof p(c, kPhaseTrsm, (double)w * w * w / 3.0, 24.0 * (double)w * w, st);
       LM_TRY(transpose_block(Ut, kNB, A11, lda, w, st));

@@ -17,7 +17,7 @@ struct Ctx;
 
 // --- context accessors (api.cu) ---------------------------------------------
 void count_launch(int n);  // process-wide kernel launch counter
-int* ctx_status(Ctx& c);        // device int[4]: error code, info, ticket, spare
+int* ctx_status(Ctx& c);        // device int[8]: error code, info, GEMM tickets (3), spare
 int ctx_num_sms(Ctx& c);
 int ctx_device(Ctx& c);
 // Grow-only device workspace owned by the context (slot 0..kWsSlots-1).
@@ -80,7 +80,8 @@ int trsv_lu(const T* LU, long long lda, int n, int nrhs, const T* DinvL, const T
 //   a_trans = false: A is m x k (lda)  | true: A^T is stored, k x m (lda)
 //   b_trans = false: B is k x n (ldb)  | true: B^T is stored, n x k (ldb)
 // lower_only: only C(i,j) with j <= i is read or written (requires m == n).
-// max_sms: SMs the persistent grid may occupy (0 = all of them).
+// sched: three ints of device memory, zero, for a product that runs beside other
+// kernels: tiles by ticket (left zero); keep_sms then keeps that many SMs clear.
 struct GemmDesc {
   int m = 0, n = 0, k = 0;
   double alpha = 1.0, beta = 0.0;
@@ -91,7 +92,8 @@ struct GemmDesc {
   double* C = nullptr;
   long long ldc = 0;
   bool a_trans = false, b_trans = false, lower_only = false;
-  int max_sms = 0;
+  int* sched = nullptr;
+  int keep_sms = 0;
 };
 int dgemm(Ctx& c, const GemmDesc& d, cudaStream_t st);
 
