@@ -109,8 +109,9 @@ __global__ void gather_rows_kernel(const T* __restrict__ B, long long ldb, int n
 //   solve  : warp h takes column h of the block, lane = row (tri_sweep);
 //   update : every thread applies the 32 solved entries to its row.
 // w = 128 with 64 columns: 86 us before (16-row blocks solved by one warp that
-// read every operand of its serial sums from shared memory), 33 us now; with 16
-// columns of a Cholesky factor in L2 86 and 23 us.
+// read every operand of its serial sums from shared memory), 17 us now, of which
+// 3 us bring the triangle in (11 us when it came through registers); 33 us with a
+// branch per step in the sweeps.
 constexpr int kTrsmLd = 129, kTrsmCols = 8;
 constexpr size_t kTrsmSmem = sizeof(double) * (128 * kTrsmLd + 128 + 2 * 32 * kTrsmCols);
 
@@ -125,18 +126,22 @@ __global__ void __launch_bounds__(256) trsm_left_kernel(const double* __restrict
   const int c0 = blockIdx.x * kTrsmCols;
   const int nc = min(kTrsmCols, ncols - c0);
   const int row = tid & 127, cg = (tid >> 7) * 4;  // this thread's row and columns of B
-  double x[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) x[c] = row < w && cg + c < nc ? B[(long long)row * ldb + c0 + cg + c] : 0.0;
-#pragma unroll 16
+  // every entry of the triangle on its way at once
   for (int r = warp; r < w; r += 8) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int c = q * 32 + lane;
       if (c < w && (lower ? c <= r : c >= r))
-        Ts[trans ? c * kTrsmLd + r : r * kTrsmLd + c] = __ldg(Tri + (long long)r * ldt + c);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                         smem_u32(Ts + (trans ? c * kTrsmLd + r : r * kTrsmLd + c))),
+                     "l"(Tri + (long long)r * ldt + c)
+                     : "memory");
     }
   }
+  double x[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) x[c] = row < w && cg + c < nc ? B[(long long)row * ldb + c0 + cg + c] : 0.0;
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   if (!unit && tid < w) dr[tid] = 1.0 / Ts[tid * kTrsmLd + tid];  // (read after the next barrier)
   const int nb = (w + 31) / 32;

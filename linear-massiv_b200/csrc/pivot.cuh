@@ -100,8 +100,8 @@ __device__ __forceinline__ T quotient(T y, T d, T r) {
 }
 
 // One triangular block of up to W rows by the W lanes of a group, lane l = row:
-// y its right-hand side, t its row of the triangle, d and r its diagonal entry and
-// the reciprocal (ignored with `unit`).  An entry leaves by shuffle as soon as it
+// y its right-hand side, t its row of the triangle (readable over bw entries, for
+// l >= bw too), d and r its diagonal entry and the reciprocal (ignored with `unit`).  An entry leaves by shuffle as soon as it
 // is final and is applied to the lanes that wait for it (the rows after it, or
 // before it when !fwd).  Branch-free with quotients by the reciprocal; where one
 // of them was not safe (see quotient) the block is solved again by divisions.
@@ -114,7 +114,7 @@ __device__ __forceinline__ T tri_sweep(T y0, const T* t, T d, T r, int l, int bw
   for (int s = 0; s < bw; ++s) {
     const int k = fwd ? s : bw - 1 - s;
     const bool waits = in && (fwd ? l > k : l < k);
-    const T tk = waits ? t[k] : T(0);
+    const T tk = t[k];  // (read whether it is used or not: a branch would split the warp)
     if (!unit) {
       pre = l == k ? y : pre;
       const T q = div_by(y, d, r);
