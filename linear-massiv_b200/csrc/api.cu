@@ -1188,7 +1188,7 @@ struct lm_batch {
   lm_ctx* ctx = nullptr;
   long long id = 0;  // unique per plan: keys its captured graphs (a freed plan's address can be reused)
   int count = 0, prec = 0;
-  int nmax = 0, rmax = 0, nbmax = 0;
+  int nmax = 0, rmax = 0;
   std::vector<long long> a_off, b_off;
   lm::BatchItem* d_items = nullptr;
   double* d_F = nullptr;
@@ -1260,11 +1260,9 @@ int batch_build(Ctx& c, lm_batch* p, int count, const int* n, const int* nrhs, c
     it.index = i;
     p->nmax = std::max(p->nmax, n[i]);
     p->rmax = std::max(p->rmax, nrhs[i]);
-    p->nbmax = std::max(p->nbmax, it.nb);
   }
   p->nmax = std::max(p->nmax, 1);
   p->rmax = std::max(p->rmax, 1);
-  p->nbmax = std::max(p->nbmax, 1);
   // longest processing time first: the largest instances are taken first so
   // the small ones fill in behind them
   auto cost = [](const lm::BatchItem& it) {
@@ -1287,7 +1285,7 @@ int batch_build(Ctx& c, lm_batch* p, int count, const int* n, const int* nrhs, c
   LM_CUDA_TRY(cudaMemset(p->d_info, 0, sizeof(int) * ni));
   LM_CUDA_TRY(cudaMemset(p->d_iters, 0, sizeof(int) * ni));
   LM_CUDA_TRY(cudaMemset(p->d_berr, 0, sizeof(double) * ni));
-  p->smem = lm::batch_smem_bytes(p->nmax, p->rmax, p->nbmax);
+  p->smem = lm::batch_smem_bytes(p->nmax, p->rmax, prec);
   if (p->smem > 200 * 1024) {
     lm::set_last_error("batch: shared memory of the largest instance exceeds 200 KB");
     return LM_ERR_UNSUPPORTED;
@@ -1307,7 +1305,6 @@ int batch_run(Ctx& c, lm_batch* p, const double* A, const double* B, double* X, 
   g.prec = p->prec;
   g.nmax = p->nmax;
   g.rmax = p->rmax;
-  g.nbmax = p->nbmax;
   g.A = A;
   g.B = B;
   g.X = X;

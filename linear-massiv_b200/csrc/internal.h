@@ -275,7 +275,7 @@ struct BatchArgs {
   const BatchItem* items;
   int count;
   int prec;             // LM_PREC_FP64 or LM_PREC_FP32_IR
-  int nmax, rmax, nbmax;
+  int nmax, rmax;
   const double* A;
   const double* B;
   double* X;
@@ -304,8 +304,8 @@ struct ServeRing {
 // Launch the device-resident loop (FP64 solves of the posted requests).
 int serve_loop_launch(const BatchArgs& g, const ServeRing& rg, int grid, size_t smem, cudaStream_t st);
 
-// Dynamic shared memory of the batch kernel for the given maxima.
-size_t batch_smem_bytes(int nmax, int rmax, int nbmax);
+// Dynamic shared memory of the batch kernel for the given maxima and precision.
+size_t batch_smem_bytes(int nmax, int rmax, int prec);
 // Resident CTAs per SM of the batch kernel at that shared-memory size.
 int batch_occupancy(size_t smem, int* per_sm);
 // Reset the ticket and launch `grid` persistent CTAs on `st`.

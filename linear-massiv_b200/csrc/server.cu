@@ -364,7 +364,6 @@ void lane_run(Lane* ln) {
     const double t0 = now_s();
     char* base = s->arena.base;
     int nmax = 1, rmax = 1;
-    int nbmax = 1;
     int err = LM_OK;
     const int k = (int)jobs.size();
     for (int i = 0; i < k && err == LM_OK; ++i) {
@@ -387,7 +386,6 @@ void lane_run(Lane* ln) {
       it.index = i;
       nmax = std::max(nmax, r->n);
       rmax = std::max(rmax, r->nrhs);
-      nbmax = std::max(nbmax, it.nb);
     }
     // largest first within the micro-batch
     std::sort(ln->h_items, ln->h_items + k, [](const lm::BatchItem& a, const lm::BatchItem& b) {
@@ -403,7 +401,6 @@ void lane_run(Lane* ln) {
       g.prec = s->cfg.small_precision;
       g.nmax = nmax;
       g.rmax = rmax;
-      g.nbmax = nbmax;
       g.A = reinterpret_cast<const double*>(base);
       g.B = reinterpret_cast<const double*>(base);
       g.X = reinterpret_cast<double*>(base);
@@ -415,7 +412,7 @@ void lane_run(Lane* ln) {
       g.ticket = ln->d_ticket;
       g.tol = 0.0;
       g.max_iter = 10;
-      const size_t smem = lm::batch_smem_bytes(nmax, rmax, nbmax);
+      const size_t smem = lm::batch_smem_bytes(nmax, rmax, s->cfg.small_precision);
       int per_sm = 1;
       err = lm::batch_occupancy(smem, &per_sm);
       const int grid = std::max(1, std::min(k, std::max(per_sm, 1) * s->num_sms));
@@ -542,7 +539,6 @@ lm::BatchArgs loop_args(lm_server* s) {
   g.prec = LM_PREC_FP64;
   g.nmax = std::max(1, s->cfg.small_max_n);
   g.rmax = 16;
-  g.nbmax = 32;
   g.A = reinterpret_cast<const double*>(base);
   g.B = reinterpret_cast<const double*>(base);
   g.X = reinterpret_cast<double*>(base);
@@ -858,13 +854,13 @@ int server_init(lm_server* s) {
   }
   // the batch kernel's shared-memory limit for the largest micro-batch shape
   int per_sm = 0;
-  LM_TRY(lm::batch_occupancy(lm::batch_smem_bytes(s->cfg.small_max_n, 16, 32), &per_sm));
+  LM_TRY(lm::batch_occupancy(lm::batch_smem_bytes(s->cfg.small_max_n, 16, s->cfg.small_precision), &per_sm));
   if (s->cfg.device_loop) {
     DeviceLoop* L = new DeviceLoop;
     s->loop = L;
     L->cap = 8192;
     L->ctas = std::max(1, std::min(s->cfg.loop_ctas, s->num_sms));
-    L->smem = lm::batch_smem_bytes(std::max(1, s->cfg.small_max_n), 16, 32);
+    L->smem = lm::batch_smem_bytes(std::max(1, s->cfg.small_max_n), 16, LM_PREC_FP64);
     L->posted.assign(L->cap, nullptr);
     L->seq_of.assign(L->cap, -1);
     LM_CUDA_TRY(cudaStreamCreateWithFlags(&L->feed, cudaStreamNonBlocking));
