@@ -317,14 +317,15 @@ int dgetrs(Ctx& c, int n, int nrhs, const double* LU, long long lda, const int* 
   if (nrhs <= 4) {
     // few right-hand sides: P b, then one persistent launch per direction
     void* ws = nullptr;
-    LM_TRY(ctx_workspace(c, 2, 64 + sizeof(double) * (size_t)n * nrhs, &ws));
+    const size_t sync_bytes = trsv_sync_bytes<double>(n, nrhs);
+    LM_TRY(ctx_workspace(c, 2, sync_bytes + sizeof(double) * (size_t)n * nrhs, &ws));
     {
       Prof p(c, kPhaseSwap, 0.0, 32.0 * n * nrhs, st);
-      LM_TRY(laswp_narrow<double>(B, ldb, n, nrhs, ipiv, reinterpret_cast<double*>(static_cast<char*>(ws) + 64),
+      LM_TRY(laswp_narrow<double>(B, ldb, n, nrhs, ipiv, reinterpret_cast<double*>(static_cast<char*>(ws) + sync_bytes),
                                   ctx_status(c), st));
     }
     Prof p(c, kPhaseTrsm, 2.0 * n * n * nrhs, 8.0 * n * n, st);
-    return trsv_lu<double>(LU, lda, n, nrhs, nullptr, nullptr, B, ldb, static_cast<int*>(ws), ctx_status(c), st);
+    return trsv_lu<double>(LU, lda, n, nrhs, nullptr, nullptr, B, ldb, ws, ctx_status(c), st);
   }
   SolveBufs sb;
   LM_TRY(solve_bufs(c, n, nrhs, LU, lda, B, ldb, n, sb, st));
@@ -368,15 +369,15 @@ int dpotrs(Ctx& c, int n, int nrhs, const double* G, long long lda, double* B, l
     // stored diagonal of G)
     const long long ldp = (n + 7) / 8 * 8;
     void* ws = nullptr;
-    LM_TRY(ctx_workspace(c, 2, 256 + sizeof(double) * (size_t)n * ldp, &ws));
-    int* sync = static_cast<int*>(ws);
-    double* P = reinterpret_cast<double*>(static_cast<char*>(ws) + 256);
+    const size_t sync_bytes = trsv_sync_bytes<double>(n, nrhs);
+    LM_TRY(ctx_workspace(c, 2, sync_bytes + sizeof(double) * (size_t)n * ldp, &ws));
+    double* P = reinterpret_cast<double*>(static_cast<char*>(ws) + sync_bytes);
     {
       Prof p(c, kPhaseOther, 0.0, 16.0 * n * n, st);
       LM_TRY(pack_lower_sym(P, ldp, G, lda, n, st));
     }
     Prof p(c, kPhaseTrsm, 2.0 * n * n * nrhs, 8.0 * n * n, st);
-    return trsv_lu<double>(P, ldp, n, nrhs, nullptr, nullptr, B, ldb, sync, ctx_status(c), st, nullptr, true, false);
+    return trsv_lu<double>(P, ldp, n, nrhs, nullptr, nullptr, B, ldb, ws, ctx_status(c), st, nullptr, true, false);
   }
   SolveBufs sb;
   LM_TRY(solve_bufs(c, n, nrhs, G, lda, B, ldb, 0, sb, st));

@@ -70,9 +70,12 @@ int tri_inv_blocks(const T* LU, long long lda, int n, T* DinvL, T* DinvU, cudaSt
 // correction step to flagged blocks.
 // unit_lower = false reads L's stored diagonal (a Cholesky factor G packed
 // with G^T above the diagonal).
+// Bytes of `sync` for n rows and nrhs right-hand sides.
+template <typename T>
+size_t trsv_sync_bytes(int n, int nrhs);
 template <typename T>
 int trsv_lu(const T* LU, long long lda, int n, int nrhs, const T* DinvL, const T* DinvU, T* X, long long ldx,
-            int* sync, int* status, cudaStream_t st, const int* corr = nullptr, bool exact = false,
+            void* sync, int* status, cudaStream_t st, const int* corr = nullptr, bool exact = false,
             bool unit_lower = true);
 
 // --- FP64 GEMM (dgemm.cu) ----------------------------------------------------

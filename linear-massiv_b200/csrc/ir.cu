@@ -612,7 +612,7 @@ int dgesv_ir(Ctx& c, int n, int nrhs, const double* A, long long lda, const doub
   const size_t r_bytes = sizeof(double) * (size_t)n * ldr;
   const size_t d_bytes = sizeof(float) * (size_t)n * ldr;
   const size_t nrm_bytes = sizeof(unsigned long long) * (size_t)(2 + 3 * 64);  // 16-byte multiple
-  const size_t sync_bytes = 64;
+  const size_t sync_bytes = trsv_sync_bytes<float>(n, nrhs);
   const size_t w_bytes = sizeof(float) * (size_t)n * ldr;  // gather scratch of the interchanges
   // GMRES-IR (low-precision factors): Krylov bases V (M + 1) and Z (M), W, a
   // zero block, dot-product partials and coefficients
@@ -632,7 +632,7 @@ int dgesv_ir(Ctx& c, int n, int nrhs, const double* A, long long lda, const doub
   double* R = reinterpret_cast<double*>(p + a32_bytes + piv_bytes);
   float* D = reinterpret_cast<float*>(p + a32_bytes + piv_bytes + r_bytes);
   unsigned long long* nrm = reinterpret_cast<unsigned long long*>(p + a32_bytes + piv_bytes + r_bytes + d_bytes);
-  int* tsync = reinterpret_cast<int*>(p + a32_bytes + piv_bytes + r_bytes + d_bytes + nrm_bytes);
+  void* tsync = static_cast<void*>(p + a32_bytes + piv_bytes + r_bytes + d_bytes + nrm_bytes);
   float* Wg = reinterpret_cast<float*>(p + a32_bytes + piv_bytes + r_bytes + d_bytes + nrm_bytes + sync_bytes);
   if (nrhs > 64) return LM_ERR_UNSUPPORTED;
   GmresBufs gb{};
@@ -872,7 +872,7 @@ int dgesv_rbt_ir(Ctx& c, int n, int nrhs, const double* A, long long lda, const 
   const size_t inv_elems = trsv_inv_elems<float>(np);
   const size_t inv_bytes = 2 * sizeof(float) * inv_elems;
   const size_t diag_bytes = 4 * sizeof(double) * (size_t)np;
-  const size_t sync_bytes = 64;
+  const size_t sync_bytes = trsv_sync_bytes<float>(np, nrhs);
   const size_t flag_bytes = sizeof(int) * 2 * (size_t)((np + 127) / 128);
   void* ws = nullptr;
   LM_TRY(ctx_workspace(c, 0, a32_bytes + r_bytes + d_bytes + nrm_bytes + inv_bytes + diag_bytes + sync_bytes + flag_bytes,
@@ -892,7 +892,7 @@ int dgesv_rbt_ir(Ctx& c, int n, int nrhs, const double* A, long long lda, const 
   double* du = reinterpret_cast<double*>(p);
   double* dv = du + 2 * (size_t)np;
   p += diag_bytes;
-  int* tsync = reinterpret_cast<int*>(p);
+  void* tsync = static_cast<void*>(p);
   p += sync_bytes;
   int* rflag = reinterpret_cast<int*>(p);
   LM_TRY(input_norms(n, nrhs, A, lda, B, ldb, nrm, nrm_bytes, st));
