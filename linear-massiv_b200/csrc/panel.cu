@@ -807,7 +807,6 @@ int panel_lu(Ctx& c, T* A, long long lda, int n, int c0, int pw, int* ipiv, int*
   return LM_ERR_UNSUPPORTED;
 }
 
-template int panel_ctas<double>(Ctx&, int);
 template int panel_ctas<float>(Ctx&, int);
 template int panel_lu<double>(Ctx&, double*, long long, int, int, int, int*, int*, cudaStream_t);
 template int panel_lu<float>(Ctx&, float*, long long, int, int, int, int*, int*, cudaStream_t);
