@@ -34,8 +34,9 @@
 // solves run in FP32; the solution is refined in FP64 inside the same CTA —
 // r = B - A X with the original FP64 A (DMMA), correction from the FP32 factors,
 // X += D — until the normwise backward error max_h ||r_h|| / (||A|| ||x_h|| +
-// ||b_h||) (infinity norms) is <= tol.  An instance that has not converged
-// after max_iter corrections is refactored and solved in FP64 (iters = -1).
+// ||b_h||) (infinity norms) is <= tol, which a column with a NaN or an infinity in
+// any of these norms never is.  An instance that has not converged after max_iter
+// corrections is refactored and solved in FP64 (iters = -1).
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -681,16 +682,17 @@ __device__ __forceinline__ void run_fp64(const BatchItem& it, const BatchArgs& g
       [&](int i, int h, double x) { X[i * r + h] = x; });
 }
 
-// Column maxima of |get(i, h)| over n rows into red (by warp); NaN as DBL_MAX.
+// Norms of the refinement: a NaN counts as infinity, which fmax keeps where it
+// would drop the NaN.
+__device__ __forceinline__ double norm_abs(double v) { return v != v ? INFINITY : fabs(v); }
+
+// Column maxima of |get(i, h)| over n rows into red (by warp).
 template <typename Get>
 __device__ __forceinline__ void col_max(int n, int r, double (*red)[kMaxR], Get get) {
   const int h = tid_() & 15;
   double m = 0.0;
   if (h < r)
-    for (int i = tid_() >> 4; i < n; i += kBT / 16) {
-      const double v = fabs(get(i, h));
-      m = fmax(m, v != v ? DBL_MAX : v);
-    }
+    for (int i = tid_() >> 4; i < n; i += kBT / 16) m = fmax(m, norm_abs(get(i, h)));
   __syncwarp();
   m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 16));
   if ((tid_() & 31) < kMaxR) red[tid_() >> 5][h] = m;
@@ -736,7 +738,7 @@ __device__ __forceinline__ void batch_residual(const double* A, const double* B,
         if (i < n && h < r) {
           const double res = B[i * r + h] - acc[ni][e];
           D[i * r + h] = (float)res;
-          mx[ni][e & 1] = fmax(mx[ni][e & 1], res != res ? DBL_MAX : fabs(res));
+          mx[ni][e & 1] = fmax(mx[ni][e & 1], norm_abs(res));
         }
       }
   }
@@ -782,7 +784,7 @@ __device__ int run_ir(const BatchItem& it, const BatchArgs& g, unsigned char* sm
       __syncwarp();
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      m = fmax(m, s != s ? DBL_MAX : s);
+      m = fmax(m, norm_abs(s));
     }
     if (lane == 0) fx->red[0][warp][0] = m;
     col_max(n, r, fx->red[1], [&](int i, int h) { return B[i * r + h]; });
@@ -819,8 +821,9 @@ __device__ int run_ir(const BatchItem& it, const BatchArgs& g, unsigned char* sm
       if (lane < r) {
         const double rn = red_max(fx->red[0], lane);
         const double den = fx->anorm * red_max(fx->red[1], lane) + fx->bnorm[lane];
-        bh = den > 0.0 ? rn / den : (rn > 0.0 ? DBL_MAX : 0.0);
-        if (bh != bh) bh = DBL_MAX;
+        // a residual or a denominator that is not finite says nothing: never converged
+        // (rn / inf would be a perfect zero)
+        bh = rn <= DBL_MAX && den <= DBL_MAX ? (den > 0.0 ? rn / den : (rn > 0.0 ? DBL_MAX : 0.0)) : DBL_MAX;
       }
       __syncwarp();
 #pragma unroll

@@ -112,3 +112,33 @@ def test_nan_and_ties():
     assert np.array_equal(P[:40], O.lu_solve_p(A0, B[0][:, 0])[2])
     assert np.array_equal(P[40:], O.lu_solve_p(A1, B[1][:, 0])[2])
     assert np.isfinite(X[0]).all()
+
+
+def test_refinement_never_accepts_what_is_not_finite():
+    # entries beyond FP32's range, NaN and infinities beside ordinary systems: the former
+    # must come from the FP64 fallback, the latter must not be reported as converged
+    g = philox(8400)
+    m, r = 40, 3
+    plain = g.uniform(-1, 1, (m, m)) + 4 * np.eye(m)
+    spd = plain @ plain.T + m * np.eye(m)
+    spd = 0.5 * (spd + spd.T)
+    rhs = g.uniform(-1, 1, (m, r))
+    bad_a, bad_b, inf_a, inf_b = plain.copy(), rhs.copy(), plain.copy(), rhs.copy()
+    bad_a[7, 3], bad_b[5, 1], inf_a[2, 9], inf_b[11, 2] = np.nan, np.nan, np.inf, -np.inf
+    cases = [(plain, rhs, 0, "refined"), (plain * 1e39, rhs, 0, "fp64"), (spd, rhs, 1, "refined"),
+             (spd * 1e39, rhs, 1, "fp64"), (plain, rhs * 1e39, 0, "fp64"), (spd, rhs * 1e39, 1, "fp64"),
+             (bad_a, rhs, 0, "never"), (plain, bad_b, 0, "never"), (spd, bad_b, 1, "never"),
+             (inf_a, rhs, 0, "never"), (plain, inf_b, 0, "never"), (spd, inf_b, 1, "never"),
+             (plain, rhs, 0, "refined")]
+    A, B = [c[0] for c in cases], [c[1] for c in cases]
+    plan = lmb200.Batch(np.full(len(cases), m, np.int32), np.full(len(cases), r, np.int32),
+                        np.array([c[2] for c in cases], np.int32), lmb200.PREC_FP32_IR)
+    X = solve(plan, A, B)
+    info, iters, berr = plan.results()
+    for i, (a, b, _, want) in enumerate(cases):
+        if want == "refined":
+            assert info[i] == 0 and iters[i] >= 0 and berr[i] <= 1e-15 * m, i
+        else:
+            assert iters[i] == -1 and not berr[i] <= 1e-15 * m, (i, iters[i], berr[i])
+        if want != "never":
+            assert info[i] == 0 and backward(a, X[i], b).max() <= 1e-15 * m, i
