@@ -233,6 +233,18 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, WM, MINB, CSM>::THREADS, MINB)
   const uint32_t sA32 = smem_u32(sA);
   const uint32_t sB32 = smem_u32(sB);
 
+  // Gives a buffer back to the producer when every value that the warp read from it
+  // is in registers.  An arrive that merely follows the loads in program order was
+  // seen to overtake them when other warps' epilogues filled the memory pipe (the
+  // loads' users can be scheduled after it), and the next TMA load then overwrote
+  // what they were still to read.  So the arrive's address depends on a vote of
+  // all lanes over all their values: no load's order or return is taken for granted.
+  // g.zero is 0, which the compiler does not know.
+  auto give_back = [&](uint64_t* bar, uint32_t read) {
+    const int off = __any_sync(0xffffffffu, (read & g.zero) != 0u);  // 0
+    if (lane == 0) mbar_arrive(bar + off);
+  };
+
   int it = 0;
   for (int cj = 0;; ++cj) {
     if (!mbar_wait(&full[it % STAGES], (uint32_t)((it / STAGES) & 1), g.status)) return;
@@ -257,7 +269,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, WM, MINB, CSM>::THREADS, MINB)
       __syncwarp();
       const uint32_t aBase = sA32 + s * Cfg::A_BYTES;
       const uint32_t bBase = sB32 + s * Cfg::B_BYTES;
-      uint32_t read = 0;  // depends on the last operands read from the slot
+      uint32_t read = 0;  // depends on every operand read from the slot
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         double af[MI][2], bf[4];
@@ -285,20 +297,12 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, WM, MINB, CSM>::THREADS, MINB)
         for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
           for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
-        if (kk == 3) {
 #pragma unroll
-          for (int mi = 0; mi < MI; ++mi) read |= __double2hiint(af[mi][0]) | __double2hiint(af[mi][1]);
+        for (int mi = 0; mi < MI; ++mi) read |= __double2hiint(af[mi][0]) | __double2hiint(af[mi][1]);
 #pragma unroll
-          for (int ni = 0; ni < 4; ++ni) read |= __double2hiint(bf[ni]);
-        }
+        for (int ni = 0; ni < 4; ++ni) read |= __double2hiint(bf[ni]);
       }
-      __syncwarp();
-      // The slot is given back only when its operands are in registers: an arrive
-      // that merely follows the loads in program order was seen to overtake them
-      // when other warps' epilogues filled the memory pipe (their products can be
-      // scheduled after it), and the next tile's TMA then overwrote them.  g.zero
-      // is 0, which the compiler does not know.
-      if (lane == 0) mbar_arrive(&empty[s] + (read & g.zero));
+      give_back(&empty[s], read);
     }
 
     // ---------------- epilogue: C = alpha*acc + beta*C ----------------
@@ -309,6 +313,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, WM, MINB, CSM>::THREADS, MINB)
       if (!mbar_wait(cfull, (uint32_t)(cj & 1), g.status)) return;
       __syncwarp();
       const uint32_t sC32 = smem_u32(sC);
+      uint32_t read = 0;  // depends on every element read from the staged tile
 #pragma unroll
       for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
@@ -322,6 +327,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, WM, MINB, CSM>::THREADS, MINB)
             asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
                          : "=d"(o.x), "=d"(o.y)
                          : "r"(sC32 + (cl >> 4) * C_BOX + swz128(rl, cl & 15)));
+            read |= __double2hiint(o.x) | __double2hiint(o.y);
             if (row >= g.m) continue;
             const int col = tn * BN + cl;
             const bool in0 = col < g.n && (!g.lower_only || col <= row);
@@ -338,7 +344,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, WM, MINB, CSM>::THREADS, MINB)
           }
         }
       __syncwarp();
-      if (lane == 0) mbar_arrive(cempty);
+      give_back(cempty, read);
     } else {
 #pragma unroll
       for (int mi = 0; mi < MI; ++mi) {

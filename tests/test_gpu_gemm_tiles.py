@@ -38,3 +38,23 @@ def test_repeats_bitwise(ctx, m, n, k):
         lmb200.dgemm(1.0, A, B, 1.0, D, ctx)
         ref = D if ref is None else ref
         assert torch.equal(D, ref), f"run {i}: {int((D != ref).sum())} entries differ"
+
+
+@pytest.mark.parametrize("k", [4, 16, 48])
+def test_staged_c_repeats_bitwise(ctx, k):
+    # one to three k-slices per tile: the staged C tile and the ring slots are given back
+    # and refilled as fast as they can be, many tiles per CTA
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(k)
+    A, B, C = (torch.rand(s, dtype=torch.float64, device="cuda", generator=gen) for s in ((3000, k), (k, 3002), (3000, 3002)))
+    ref = None
+    for i in range(60):
+        D = C.clone()
+        if i % 3 == 0:
+            A @ B
+        lmb200.dgemm(-1.0, A, B, 1.0, D, ctx)
+        ref = D if ref is None else ref
+        assert torch.equal(D, ref), f"run {i}: {int((D != ref).sum())} entries differ"
+    exact = C - A @ B
+    # |fl - exact| <= gamma_(k+2) (|A||B| + |C|) for either of two orders; all entries are positive
+    assert bool(((ref - exact).abs() <= 2 * (k + 2) * EPS * (A @ B + C)).all())
