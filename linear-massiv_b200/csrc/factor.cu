@@ -93,7 +93,7 @@ int dgetrf(Ctx& c, int n, double* A, long long lda, int* ipiv, cudaStream_t st) 
     const int* pl = plan[(k0 / kNB) & 1];
     auto rows = [&](int ca0, int ca1, int cb0, int cb1) {
       Prof p(c, kPhaseTrsm, (double)w * w * (cb1 - cb0), 8.0 * (4.0 * w * (ca1 - ca0 + cb1 - cb0) + 0.5 * w * w), st);
-      return row_block<double>(A, lda, pl, k0, w, ca0, ca1, cb0, cb1, st);
+      return row_block<double>(A, lda, pl, n, k0, w, ca0, ca1, cb0, cb1, ctx_status(c), st);
     };
     if (m <= 0) {
       LM_TRY(rows(0, k0, n, n));

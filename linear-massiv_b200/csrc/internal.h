@@ -110,9 +110,11 @@ constexpr int kSwapPlanInts = 1 + 2 * kSwapPlanRows + 15;
 // `plan` moved on columns [ca0, ca1) and [cb0, cb1), and on [cb0, cb1) the
 // block solve  A[k0 : k0 + w, cb0 : cb1) <- inv(L11) A[...]  with the unit
 // lower triangle of the panel's diagonal block (already in its final order).
+// A row of the plan outside [k0, n) is left out and recorded as LM_DEVERR_BOUNDS
+// in status[0].
 template <typename T>
-int row_block(T* A, long long lda, const int* plan, int k0, int w, int ca0, int ca1, int cb0, int cb1,
-              cudaStream_t st);
+int row_block(T* A, long long lda, const int* plan, int n, int k0, int w, int ca0, int ca1, int cb0, int cb1,
+              int* status, cudaStream_t st);
 
 // All interchanges ipiv[0..n) on a narrow n x nrhs block B at once (one
 // parallel gather into W, n x nrhs scratch, then copied back).

@@ -258,7 +258,7 @@ int sgetrf(Ctx& c, int n, float* A, long long lda, int* ipiv, cudaStream_t st, i
     const int* pl = s.plan[(k0 / kNB) & 1];
     auto rows = [&](int ca0, int ca1, int cb0, int cb1) {
       Prof p(c, kPhaseTrsm, (double)w * w * (cb1 - cb0), 4.0 * (4.0 * w * (ca1 - ca0 + cb1 - cb0) + 0.5 * w * w), st);
-      return row_block<float>(A, lda, pl, k0, w, ca0, ca1, cb0, cb1, st);
+      return row_block<float>(A, lda, pl, n, k0, w, ca0, ca1, cb0, cb1, ctx_status(c), st);
     };
     if (m <= 0) {
       LM_TRY(rows(0, k0, n, n));

@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
 #pragma unroll 1
     for (int m0 = 0; m0 < w; m0 += MW) {
       const int wm = min(MW, w - m0);
-      if (ZW > 0 && C > 1 && tid == 0) mbar_arrive_expect_tx(&bars[2], (uint32_t)(wm * ZW * sizeof(T)));
+      if (ZW > 0 && C > 1 && tid == 0 && !timed_out) mbar_arrive_expect_tx(&bars[2], (uint32_t)(wm * ZW * sizeof(T)));
       // this thread's best candidate for the next column
       Key bk = 0;
       int bi = INT_MAX, bs = 0;
@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
           for (int s = 0; s < RPT; ++s)
             if (s == bs) vec_store<T, MW>(out->v, y[s]);
         }
-        if (C > 1 && tid == 0) mbar_arrive_expect_tx(&bars[par], (uint32_t)(C * sizeof(Msg)));
+        // (not again on a phase that did not end: its arrival is spent)
+        if (C > 1 && tid == 0 && !timed_out) mbar_arrive_expect_tx(&bars[par], (uint32_t)(C * sizeof(Msg)));
         __syncthreads();
         const int wo = warp_winner(lane < nw ? wms[lane].key : Key(0), lane < nw ? wms[lane].label : INT_MAX);
         const Msg* win = wms + wo;
@@ -429,9 +430,8 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
         } else if (j > 0) {
           send_z(j - 1, m0);
         }
-        // (row J itself is always a candidate, so some CTA wins; the fallback
-        // only keeps the indexing in bounds)
-        const int p = win->label == INT_MAX ? J : win->label;
+        // (row J itself is always a candidate, so some CTA wins)
+        const int p = pivot_position(win->label, J, timed_out);
         const T rcp = win->rcp;
         T u[MW];
         vec_load<T, MW>(u, win->v);
@@ -464,8 +464,9 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
         //      rewritten later), from where they go out beside the next exchange ----
         if constexpr (ZW > 0) {
           if (qw == q && warp == wo) {  // uniform in the warp
+            const int prow = min(bs_out * NT + tid, rpc - 1);  // (a winner has a row; see pivot_position)
             if (owner) {
-              T* sr = slab + (bs_out * NT + tid) * SLD + m0 + MW;
+              T* sr = slab + prow * SLD + m0 + MW;
 #pragma unroll
               for (int s = 0; s < RPT; ++s)
                 if (s == bs_out) {
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
                 }
             }
             __syncwarp();
-            zpush = __shfl_sync(0xffffffffu, bs_out * NT + tid, wl);
+            zpush = __shfl_sync(0xffffffffu, prow, wl);
           }
         }
         // L11 and the pivot's place, for the solves; the swap list
@@ -640,6 +641,12 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
     cluster_arrive();
     arrived = true;
   }
+
+  // After a wait that gave up the result is void (status 0 says so), the labels are
+  // still rows of the panel (pivot_position), and messages may be on their way: no
+  // CTA leaves the cluster before they have had a millisecond to land.
+  if (timed_out)
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
 
   // ---- the rows that change place: list them, then move the panel's own
   //      columns, a share of the columns per CTA ----

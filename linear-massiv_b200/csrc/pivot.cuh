@@ -2,6 +2,8 @@
 // pivot order of the reference's scan and quotients by a known reciprocal.
 #pragma once
 
+#include <climits>
+
 #include "common.cuh"
 
 namespace lm {
@@ -77,6 +79,13 @@ __device__ __forceinline__ int warp_winner(unsigned long long key, int label) {
     }
   }
   return __ffs(b) - 1;
+}
+
+// The row that takes position J of a panel, from the label of the winning
+// candidate: J itself where there is none (INT_MAX), and after a wait that gave up
+// (the message's place then holds whatever was there).
+__host__ __device__ inline int pivot_position(int label, int J, bool gave_up) {
+  return gave_up || label == INT_MAX ? J : label;
 }
 
 // x / p for a pivot p whose correctly rounded reciprocal is r: the quotient

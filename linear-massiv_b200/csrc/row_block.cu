@@ -54,8 +54,8 @@ __device__ __forceinline__ void load_l(T* buf, const T* L, long long lda, int r0
 
 template <typename T>
 __global__ void __launch_bounds__(kRbThreads, 2)
-    row_block_kernel(T* A, long long lda, const int* __restrict__ plan, int k0, int w, int ca0, int ca1, int cb0,
-                     int cb1, int ablocks) {
+    row_block_kernel(T* A, long long lda, const int* __restrict__ plan, int n, int k0, int w, int ca0, int ca1, int cb0,
+                     int cb1, int ablocks, int* status) {
   using Cfg = RbCfg<T>;
   extern __shared__ __align__(16) unsigned char sm[];
   T* X = reinterpret_cast<T*>(sm);
@@ -80,7 +80,10 @@ __global__ void __launch_bounds__(kRbThreads, 2)
   const int m = min(__ldg(plan), kSwapPlanRows);
   for (int e = tid; e < m; e += kRbThreads) {
     const int d = __ldg(plan + 1 + e), s = __ldg(plan + 1 + kSwapPlanRows + e);
-    if (d < k0 + w) {
+    // the panel moves rows [k0, n) only: anything else is recorded and left out
+    if (min(d, s) < k0 || max(d, s) >= n) {
+      atomicCAS(status, 0, LM_DEVERR_BOUNDS);
+    } else if (d < k0 + w) {
       src[d - k0] = s;
     } else {
       const int at = atomicAdd(&others, 1);  // a displaced row comes from the block: at most w of them
@@ -210,8 +213,8 @@ __global__ void __launch_bounds__(kRbThreads, 2)
 }  // namespace
 
 template <typename T>
-int row_block(T* A, long long lda, const int* plan, int k0, int w, int ca0, int ca1, int cb0, int cb1,
-              cudaStream_t st) {
+int row_block(T* A, long long lda, const int* plan, int n, int k0, int w, int ca0, int ca1, int cb0, int cb1,
+              int* status, cudaStream_t st) {
   if (w <= 0) return LM_OK;
   if (w > kRbMaxW) return LM_ERR_ARG;
   const int ablocks = cdiv(std::max(0, ca1 - ca0), kRbCols), bblocks = cdiv(std::max(0, cb1 - cb0), kRbCols);
@@ -225,14 +228,14 @@ int row_block(T* A, long long lda, const int* plan, int k0, int w, int ca0, int 
     LM_CUDA_TRY(cudaFuncSetAttribute(row_block_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, RbCfg<T>::SMEM));
     attr_set[dev] = true;
   }
-  row_block_kernel<T><<<ablocks + bblocks, kRbThreads, RbCfg<T>::SMEM, st>>>(A, lda, plan, k0, w, ca0, ca1, cb0, cb1,
-                                                                            ablocks);
+  row_block_kernel<T><<<ablocks + bblocks, kRbThreads, RbCfg<T>::SMEM, st>>>(
+      A, lda, plan, n, k0, w, ca0, ca1, cb0, cb1, ablocks, status);
   count_launch(1);
   LM_CUDA_TRY(cudaGetLastError());
   return LM_OK;
 }
 
-template int row_block<double>(double*, long long, const int*, int, int, int, int, int, int, cudaStream_t);
-template int row_block<float>(float*, long long, const int*, int, int, int, int, int, int, cudaStream_t);
+template int row_block<double>(double*, long long, const int*, int, int, int, int, int, int, int, int*, cudaStream_t);
+template int row_block<float>(float*, long long, const int*, int, int, int, int, int, int, int, int*, cudaStream_t);
 
 }  // namespace lm
