@@ -805,7 +805,7 @@ int lm_dgemv(lm_ctx* ctx, int m, int n, const double* A, int lda, const double* 
     if (m < 0 || n < 0) return LM_ERR_ARG;
     if (m == 0) return LM_OK;
     if (!y || (n > 0 && (!A || !x || lda < n))) return LM_ERR_ARG;
-    return lm::dgemv_exact(m, n, A, lda, x, y, c.stream);
+    return lm::dgemv_exact(c, m, n, A, lda, x, y, c.stream);
   });
 }
 
@@ -1099,7 +1099,7 @@ int lm_matvec_host(lm_ctx* ctx, int m, int n, const double* A, const double* x, 
     double* dy = dx + rup(std::max(n, 1), 8);
     LM_TRY(h2d_2d(c, dA, lda, A, n, m, n));
     if (n > 0) LM_CUDA_TRY(cudaMemcpyAsync(dx, x, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream));
-    LM_TRY(lm::dgemv_exact(m, n, dA, lda, dx, dy, c.stream));
+    LM_TRY(lm::dgemv_exact(c, m, n, dA, lda, dx, dy, c.stream));
     LM_CUDA_TRY(cudaMemcpyAsync(y, dy, sizeof(double) * m, cudaMemcpyDeviceToHost, c.stream));
     int r = lm::read_status(c, nullptr);
     return r < 0 ? r : LM_OK;

@@ -1,6 +1,6 @@
 // Kernels of the reference's adjacent entry points on the dense path:
 //
-//   gemv_exact_kernel     matvecP -> rawGemv (BLAS/Level2.hs:131-139,
+//   gemv_*_kernel         matvecP -> rawGemv (BLAS/Level2.hs:131-139,
 //                         Internal/Kernel.hs:119-134), in the reference's own
 //                         floating-point order, so results are bitwise equal:
 //                         per row, four FMA accumulators over the columns
@@ -28,7 +28,35 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// One warp per CTA, 8 rows: lane l of a quad carries accumulator l of its row.
+// The matvec has two forms (see gemv_short_rows); lane l of a quad carries
+// accumulator l of its row, and lane 0 ends the row in the reference's order.
+__device__ __forceinline__ void gemv_row_end(double acc, bool on, int n, const double* ar, const double* x, double* y) {
+  __syncwarp();
+  const double a1 = __shfl_down_sync(kFull, acc, 1, 4);
+  const double a2 = __shfl_down_sync(kFull, acc, 2, 4);
+  const double a3 = __shfl_down_sync(kFull, acc, 3, 4);
+  if (on && (threadIdx.x & 3) == 0) {
+    double s = __dadd_rn(__dadd_rn(__dadd_rn(acc, a1), a2), a3);
+    for (int j = n - n % 4; j < n; ++j) s = __dadd_rn(s, __dmul_rn(ar[j], x[j]));
+    *y = s;
+  }
+}
+
+// Short rows, or rows that fill the chip: 512 rows per SM at a time, each quad
+// loading as it goes (bound by the loads in flight, 8 per thread).
+__global__ void __launch_bounds__(256) gemv_rows_kernel(int m, int n, const double* __restrict__ A, long long lda,
+                                                        const double* __restrict__ x, double* __restrict__ y) {
+  const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+  const bool on = row < m;
+  const double* ar = A + (on ? row : 0) * lda;
+  const int n4 = n - n % 4;
+  double acc = 0.0;
+#pragma unroll 8
+  for (int j = threadIdx.x & 3; j < n4; j += 4) acc = fma(ar[j], x[j], acc);
+  gemv_row_end(acc, on, n, ar, x, y + row);
+}
+
+// Otherwise: one warp per CTA, 8 rows.
 // What bounds it is the bytes in flight: the four chains of a row are serial, so
 // a thread that loads as it goes has 8 loads of 8 bytes out (1.3 TB/s).  Here
 // each warp keeps kGemvStages chunks of 8 x 64 elements on their way through
@@ -90,17 +118,7 @@ __global__ void __launch_bounds__(32) gemv_exact_kernel(int m, int n, const doub
       for (int s = 0; s < steps; ++s) acc = fma(sa[4 * s], xs[4 * s], acc);
     }
   }
-  __syncwarp();
-  // lane 0 of the quad gathers the four accumulators in the reference's order
-  const double a1 = __shfl_down_sync(kFull, acc, 1, 4);
-  const double a2 = __shfl_down_sync(kFull, acc, 2, 4);
-  const double a3 = __shfl_down_sync(kFull, acc, 3, 4);
-  if (r < rows && l == 0) {
-    const double* ar = Ab + (long long)r * lda;
-    double s = __dadd_rn(__dadd_rn(__dadd_rn(acc, a1), a2), a3);
-    for (int j = n4; j < n; ++j) s = __dadd_rn(s, __dmul_rn(ar[j], x[j]));
-    y[row0 + r] = s;
-  }
+  gemv_row_end(acc, r < rows, n, Ab + (long long)(r < rows ? r : 0) * lda, x, y + row0 + r);
 }
 
 // 32 rows per CTA; column chunks of 128 staged through shared memory so the
@@ -274,8 +292,27 @@ int grid_for(long long total, int per) { return (int)std::max<long long>(1, std:
 
 }  // namespace
 
-int dgemv_exact(int m, int n, const double* A, long long lda, const double* x, double* y, cudaStream_t st) {
+// Rows for gemv_rows_kernel.  Its quads read 32 bytes of a row at a time, so a chip
+// full of them streams at 5.2 to 6 TB/s, but a last wave that is half empty, or few
+// rows, leave it without loads in flight; and a CTA of the staged kernel costs
+// its start-up per 8 rows, which short rows do not repay.  us, rows / staged:
+//   1000000 x 3 19 / 90, x 16 36 / 122, x 64 89 / 135, x 128 171 / 206;
+//   524288 x 256 189 / 221, x 1024 723 / 823; 65536 x 256 32 / 34, x 1024 110 / 110,
+//   x 2048 218 / 206; 100000 (1.3 waves) x 128 23 / 25, x 192 39 / 36, x 512 92 / 83.
+static bool gemv_short_rows(int m, int n, int sms) {
+  if (n <= 128) return true;
+  const long long wave = 512LL * sms, waves = cdivll(m, wave);
+  return n <= 1024 && 20LL * m >= 17 * waves * wave;  // (waves 85% full)
+}
+
+int dgemv_exact(Ctx& c, int m, int n, const double* A, long long lda, const double* x, double* y, cudaStream_t st) {
   if (m <= 0) return LM_OK;
+  if (gemv_short_rows(m, n, ctx_num_sms(c))) {
+    gemv_rows_kernel<<<(int)cdivll(4LL * m, 256), 256, 0, st>>>(m, n, A, lda, x, y);
+    count_launch(1);
+    LM_CUDA_TRY(cudaGetLastError());
+    return LM_OK;
+  }
   const int grid = (int)cdivll(m, kGemvRows);
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (lda & 1))
     gemv_exact_kernel<1><<<grid, 32, kGemvSmem, st>>>(m, n, A, lda, x, y);

@@ -172,7 +172,7 @@ int zero_upper(T* A, long long lda, int n, cudaStream_t st);
 
 // --- adjacent entry points (aux_solvers.cu) -----------------------------------
 // y = A x in rawGemv's floating-point order (bitwise the reference's matvecP).
-int dgemv_exact(int m, int n, const double* A, long long lda, const double* x, double* y, cudaStream_t st);
+int dgemv_exact(Ctx& c, int m, int n, const double* A, long long lda, const double* x, double* y, cudaStream_t st);
 // normInf of A (bitwise the reference's row folds) as the bits of a
 // non-negative double in *out (device).
 int dnorm_inf_exact(int m, int n, const double* A, long long lda, unsigned long long* out, cudaStream_t st);

@@ -36,3 +36,16 @@ def test_matvec_nonfinite():
     A[0, 3], A[1, 128], A[2, 129], x[64] = np.inf, np.nan, -np.inf, -0.0
     y = lmb200.matvec(torch.from_numpy(A).cuda(), torch.from_numpy(x).cuda()).cpu().numpy()
     assert np.array_equal(y, O.matvec_p(A, x), equal_nan=True)
+
+
+@pytest.mark.parametrize("m,n", [(65, 127), (65, 128), (65, 129), (8, 130),  # the short-row line
+                                 (200, 1), (1001, 7), (300, 128),
+                                 # rows that fill the chip once, its edge at 85% of a wave, a wave and a half
+                                 (75776, 129), (75776, 1024), (75776, 1025), (64409, 150), (64410, 150),
+                                 (113664, 131)])
+def test_matvec_forms(m, n):
+    g = philox(3 * m + n)
+    A = g.uniform(-1.0, 1.0, (m, n))
+    x = g.uniform(-1.0, 1.0, n)
+    y = lmb200.matvec(torch.from_numpy(A).cuda(), torch.from_numpy(x).cuda()).cpu().numpy()
+    assert np.array_equal(y, O.matvec_p(A, x))
