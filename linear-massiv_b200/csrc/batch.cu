@@ -25,8 +25,8 @@
 //            hand side), and the block column arrives by cp.async meanwhile.
 // 10,000 systems of order 8 to 256, FP64: 14.7 ms with 256-thread CTAs, panels in
 // shared memory (ten shuffles, three barriers and a serial row loop per column)
-// and row interchanges through L2, 10.2 ms now; 3,000 with FP32 factors and
-// refinement 8.25 and 4.07 ms.  What is left is latency: a warp issues every 17
+// and row interchanges through L2, 9.5 ms now; 3,000 with FP32 factors and
+// refinement 8.25 and 3.9 ms.  What is left is latency: a warp issues every 17
 // cycles, waiting at barriers (28%: the 16 x 16 diagonal blocks and the pivot
 // votes), for instructions (19%) and for fixed latencies (13%).
 //
@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.h"
@@ -406,38 +407,53 @@ __device__ void lu_factor(T* F, int n, int nb, int* ipiv, unsigned char* region,
   }
 }
 
-// The w x w diagonal block (w <= 16) at the top of P by one warp, lane = row;
-// rd receives the reciprocals of its diagonal.
+// The w x w diagonal block (w <= 16) at the top of P by one warp, lane = row; Fd
+// is the block in global memory, still as it was; rd receives the reciprocals of
+// the diagonal.  The columns are a rolled loop over rotating registers, each
+// finished one going to P at once: unrolled, the 16 steps were the largest piece of
+// code of the kernel, ran whole for the smallest block, and waited for instructions.
+// The last eight columns (all of a block of up to eight) shuffle half as much.
+// 148 SPD systems of order 4, 16, 32, 64: 21, 23, 39, 68 us unrolled, 13, 17, 31,
+// 56 us now (11, 21, 36, 70 us with a barrier per column).
 template <typename T>
-__device__ __forceinline__ void chol_diag(T* P, int w, int k0, T* rd, Fixed* fx) {
+__device__ __forceinline__ void chol_diag(T* P, const T* Fd, int n, int w, int k0, T* rd, Fixed* fx) {
   const int lane = tid_() & 31;
-  T a[kPW];
+  T a[kPW];  // slot 0 is the current column
 #pragma unroll
-  for (int c = 0; c < kPW; ++c)
-    a[c] = lane < w && c < w ? (c <= lane ? P[lane * kLdP + c] : T(0)) : (c == lane ? T(1) : T(0));
+  for (int c = 0; c < kPW; ++c) a[c] = c <= lane && lane < w ? P[lane * kLdP + c] : T(0);
   bool ok = true;
   T rj = T(0);
-  __syncwarp();  // a warp split by the loops before would serialise the shuffles
-#pragma unroll
-  for (int j = 0; j < kPW; ++j) {
-    const T d = __shfl_sync(0xffffffffu, a[j], j);
-    if (lane == 0 && j < w && !(d > T(0)) && fx->info == 0) fx->info = k0 + j + 1;
+  int j = 0;
+  auto column = [&](auto live) {  // slots in use
+    constexpr int N = decltype(live)::value;
+    __syncwarp();  // a split warp would serialise the shuffles
+    const T d = __shfl_sync(0xffffffffu, a[0], j);
+    if (lane == 0 && !(d > T(0)) && fx->info == 0) fx->info = k0 + j + 1;
     __syncwarp();
     const T s = sqrt(d), r = PivKey<T>::rcp(s);
-    ok = ok && PivKey<T>::safe(s) && (lane <= j || lane >= w || quotient_safe(a[j]));
-    const T l = div_by(a[j], s, r);
-    a[j] = lane == j ? s : (lane > j && lane < w ? l : a[j]);
+    ok = ok && PivKey<T>::safe(s) && (lane <= j || lane >= w || quotient_safe(a[0]));
+    const T q = div_by(a[0], s, r), l = lane == j ? s : q;
     rj = lane == j ? r : rj;
+    if (lane >= j && lane < w) P[lane * kLdP + j] = l;
+    __syncwarp();
+    // (rows above the entry, and lanes that hold none, are left alone: lane < j + c)
 #pragma unroll
-    for (int c = j + 1; c < kPW; ++c) {
-      const T lc = __shfl_sync(0xffffffffu, a[j], c);
-      a[c] = lane >= c ? fma(-a[j], lc, a[c]) : a[c];
+    for (int c = 1; c < N; ++c) {
+      const T lc = __shfl_sync(0xffffffffu, l, j + c);
+      a[c - 1] = lane >= j + c ? fma(-l, lc, a[c]) : a[c];
     }
-  }
+  };
+  if (w > kPW / 2)
+#pragma unroll 1
+    for (; j < kPW / 2; ++j) column(std::integral_constant<int, kPW>());
+#pragma unroll 1
+  for (; j < w; ++j) column(std::integral_constant<int, kPW / 2>());
   // a quotient by reciprocal was not safe: the same steps again with divisions
   if (!__all_sync(0xffffffffu, ok)) {
     if (lane == 0 && fx->info > k0) fx->info = 0;
-    for (int j = 0; j < w; ++j) {
+    for (int c = 0; c <= lane && lane < w; ++c) P[lane * kLdP + c] = Fd[lane * n + c];
+    __syncwarp();
+    for (j = 0; j < w; ++j) {
       const T d = P[j * kLdP + j], s = sqrt(d);
       if (lane == 0 && !(d > T(0)) && fx->info == 0) fx->info = k0 + j + 1;
       __syncwarp();
@@ -454,10 +470,6 @@ __device__ __forceinline__ void chol_diag(T* P, int w, int k0, T* rd, Fixed* fx)
   }
   if (lane == 0) fx->plain = 0;
   if (lane < kPW) rd[lane] = rj;
-  if (lane < w)
-#pragma unroll
-    for (int c = 0; c < kPW; ++c)
-      if (c <= lane) P[lane * kLdP + c] = a[c];
 }
 
 // Cholesky (lower) in place: G in the lower triangle, the strict upper
@@ -480,7 +492,7 @@ __device__ void chol_factor(T* F, int n, int nb, unsigned char* region, Fixed* f
     cp_wait<0>();
     __syncthreads();
     // (not the same warp in every CTA of an SM: those share a scheduler)
-    if ((tid_() >> 5) == (fx->slot & (kBT / 32 - 1))) chol_diag<T>(P, w, k0, rd, fx);
+    if ((tid_() >> 5) == (fx->slot & (kBT / 32 - 1))) chol_diag<T>(P, F + k0 * n + k0, n, w, k0, rd, fx);
     __syncthreads();
     for (int i = w + tid_(); i < M; i += kBT) {
       // row i: x L11^T = a, by columns of L11

@@ -142,3 +142,25 @@ def test_refinement_never_accepts_what_is_not_finite():
             assert iters[i] == -1 and not berr[i] <= 1e-15 * m, (i, iters[i], berr[i])
         if want != "never":
             assert info[i] == 0 and backward(a, X[i], b).max() <= 1e-15 * m, i
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-200])  # 1e-200: the diagonal blocks take their divisions
+@pytest.mark.parametrize("prec", [lmb200.PREC_FP64, lmb200.PREC_FP32_IR])
+def test_first_pivot_that_is_not_positive(prec, scale):
+    # L D L^T with one negative d: the Cholesky pivots are d, so info is its place, in
+    # every column of the 16-column blocks, of their halves and of ragged last blocks
+    g = philox(8500)
+    cases = [(n, p) for n in (4, 8, 9, 16, 24, 40) for p in range(n)]
+    A, B = [], []
+    for n, p in cases:
+        L = np.tril(g.uniform(-0.5, 0.5, (n, n)), -1) + np.eye(n)
+        d = g.uniform(1, 2, n)
+        d[p] = -1.5
+        M = (L * d) @ L.T
+        A.append(0.5 * (M + M.T) * scale)
+        B.append(g.uniform(-1, 1, (n, 2)))
+    plan = lmb200.Batch(np.array([n for n, _ in cases], np.int32), np.full(len(cases), 2, np.int32),
+                        np.ones(len(cases), np.int32), prec)
+    solve(plan, A, B)
+    info = plan.results()[0]
+    assert np.array_equal(info, [p + 1 for _, p in cases])
