@@ -277,9 +277,10 @@ int lm_batch_factors(const lm_batch* plan, const double** F, const int** ipiv);
 int lm_batch_solve_host(lm_batch* plan, const double* A, const double* B, double* X, double tol, int max_iter);
 /* Project-written autotuner: for each size bucket (n <= 32, 64, 128, 256)
  * times the batch kernel on a seeded synthetic batch of that bucket with each
- * candidate panel width (8, 16, 32) and keeps the fastest in the context's
+ * candidate panel width (8, 16) and keeps the fastest in the context's
  * table; `path` (may be NULL) receives the table as JSON.  lm_batch_tune_get /
- * lm_batch_tune_set read and write the table (nb[precision][bucket]). */
+ * lm_batch_tune_set read and write the table (nb[precision][bucket]: 8, 16, or
+ * 32, which runs as 16). */
 int lm_batch_tune(lm_ctx* ctx, int precision, const char* path);
 int lm_batch_tune_get(lm_ctx* ctx, int* nb /* [2][4] */);
 int lm_batch_tune_set(lm_ctx* ctx, const int* nb /* [2][4] */);
@@ -318,7 +319,7 @@ typedef struct {
   int max_batch;        /* most requests per micro-batch (default 4096) */
   int max_n;            /* largest admissible order (default 4096) */
   int max_nrhs;         /* most right-hand sides (default 64, <= 64) */
-  int nb[4];            /* batch-kernel panel width per size bucket (default 16) */
+  int nb[4];            /* batch-kernel panel width per size bucket (8, 16, or 32, which runs as 16; default 16) */
   int ir_method;        /* factorisation of the large mixed-precision solves: LM_IR_GEPP
                            (default: FP32 partial pivoting, the same result for a request
                            alone and in any mix) or LM_IR_RBT (the randomised factor

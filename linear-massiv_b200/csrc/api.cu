@@ -1448,7 +1448,7 @@ int lm_batch_tune_set(lm_ctx* ctx, const int* nb) {
 int lm_batch_tune(lm_ctx* ctx, int precision, const char* path) {
   if (!ctx || (precision != LM_PREC_FP64 && precision != LM_PREC_FP32_IR)) return LM_ERR_ARG;
   const int lo[4] = {1, 33, 65, 129}, hi[4] = {32, 64, 128, 256};
-  const int cands[3] = {8, 16, 32};
+  const int cands[2] = {8, 16};  // (the kernel's widths; 32 runs as 16)
   double best_ms[4] = {0, 0, 0, 0};
   int num_sms = 0;
   {

@@ -164,3 +164,13 @@ def test_first_pivot_that_is_not_positive(prec, scale):
     solve(plan, A, B)
     info = plan.results()[0]
     assert np.array_equal(info, [p + 1 for _, p in cases])
+
+
+def test_tuner_keeps_a_width_that_the_kernel_has():
+    ctx = lmb200.Context(0)
+    for prec in (lmb200.PREC_FP64, lmb200.PREC_FP32_IR):
+        lmb200.batch_tune_set([[32] * 4] * 2, ctx)  # accepted, and runs as 16
+        assert lmb200.batch_tune_get(ctx) == [[32] * 4] * 2
+        table = lmb200.batch_tune(prec, None, ctx)
+        assert set(table[prec]) <= {8, 16}, table
+        assert table[1 - prec] == [32] * 4
