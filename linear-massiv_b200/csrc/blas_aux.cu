@@ -196,16 +196,6 @@ __global__ void copy2d_kernel(T* dst, long long ldd, const T* src, long long lds
 }
 
 template <typename T>
-__global__ void identity_kernel(T* A, long long lda, int rows, int cols) {
-  const long long total = (long long)rows * cols;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(i / cols), c = (int)(i % cols);
-    A[(long long)r * lda + c] = (r == c) ? T(1) : T(0);
-  }
-}
-
-template <typename T>
 __global__ void zero_upper_kernel(T* A, long long lda, int n) {
   const long long total = (long long)n * n;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -310,15 +300,6 @@ int copy2d(T* dst, long long ldd, const T* src, long long lds, int rows, int col
 }
 
 template <typename T>
-int set_identity(T* A, long long lda, int rows, int cols, cudaStream_t st) {
-  if (rows <= 0 || cols <= 0) return LM_OK;
-  identity_kernel<T><<<grid_for((long long)rows * cols, 256, 148), 256, 0, st>>>(A, lda, rows, cols);
-  count_launch(1);
-  LM_CUDA_TRY(cudaGetLastError());
-  return LM_OK;
-}
-
-template <typename T>
 int zero_upper(T* A, long long lda, int n, cudaStream_t st) {
   if (n <= 1) return LM_OK;
   zero_upper_kernel<T><<<grid_for((long long)n * n, 256, 148), 256, 0, st>>>(A, lda, n);
@@ -362,13 +343,10 @@ int dresidual(Ctx& c, int n, int nrhs, const double* A, long long lda, const dou
 }
 
 template int laswp_narrow<double>(double*, long long, int, int, const int*, double*, int*, cudaStream_t);
-template int laswp_narrow<float>(float*, long long, int, int, const int*, float*, int*, cudaStream_t);
 template int laswp_perm<double>(double*, long long, int, int, const int*, double*, cudaStream_t);
 template int laswp_perm<float>(float*, long long, int, int, const int*, float*, cudaStream_t);
 template int copy2d<double>(double*, long long, const double*, long long, int, int, cudaStream_t);
 template int copy2d<float>(float*, long long, const float*, long long, int, int, cudaStream_t);
-template int set_identity<double>(double*, long long, int, int, cudaStream_t);
-template int set_identity<float>(float*, long long, int, int, cudaStream_t);
 template int zero_upper<double>(double*, long long, int, cudaStream_t);
 template int zero_upper<float>(float*, long long, int, cudaStream_t);
 

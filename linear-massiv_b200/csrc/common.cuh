@@ -14,16 +14,16 @@ namespace lm {
 // Device-side status words live in lm_ctx::d_status:
 //   [0] device error code (0 = none; LM_DEVERR_* below)
 //   [1] LAPACK-style info of the last factorisation (0 = ok, k+1 = first bad pivot)
-//   [2] scratch counter (ticket dispenser for persistent kernels)
+//   [2..4] tickets of the products that run beside a panel (dgemm.cu): zero between launches
 enum : int {
   LM_DEVERR_NONE = 0,
   LM_DEVERR_TIMEOUT = 1,   // a bounded wait gave up
   LM_DEVERR_BOUNDS = 2,    // a self-check found an out-of-range index
 };
 
-// Every spin-wait in this library gives up after this many polls, records
-// LM_DEVERR_TIMEOUT and returns.  With the hardware's own suspend inside
-// mbarrier.try_wait this bounds a wait to well under a few seconds.
+// Every spin-wait in this library gives up after this many polls (four times as many
+// where they do not suspend), records LM_DEVERR_TIMEOUT and returns: after a few
+// seconds, and up to about 20 s where polls sleep a microsecond (trsv.cu).
 constexpr uint32_t kSpinLimit = 1u << 24;
 
 struct Ctx;  // defined in api.cu
@@ -158,28 +158,6 @@ __device__ __forceinline__ uint32_t dsmem_map(const void* p, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(p)), "r"(rank));
   return out;
 }
-
-__device__ __forceinline__ double dsmem_ld_f64(uint32_t addr) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ float dsmem_ld_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ int dsmem_ld_s32(uint32_t addr) {
-  int v;
-  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
-template <typename T>
-__device__ __forceinline__ T dsmem_ld(uint32_t addr);
-template <>
-__device__ __forceinline__ double dsmem_ld<double>(uint32_t a) { return dsmem_ld_f64(a); }
-template <>
-__device__ __forceinline__ float dsmem_ld<float>(uint32_t a) { return dsmem_ld_f32(a); }
 
 // Asynchronous 16-byte store into (possibly another CTA's) shared memory that
 // completes tx bytes on the destination CTA's mbarrier (both addresses are

@@ -58,21 +58,17 @@ int make_tmap_2d(CUtensorMap* tm, CUtensorMapDataType dt, int elem_bytes, const 
 // Elements of one factor's diagonal-block inverses for order n.
 template <typename T>
 size_t trsv_inv_elems(int n);
-// DinvL / DinvU <- inverses of the diagonal blocks of the packed LU factor's
-// unit-lower L and upper U (16-byte aligned, trsv_inv_elems<T>(n) each).
+// Bytes of `sync` for n rows and nrhs right-hand sides.
 template <typename T>
-int tri_inv_blocks(const T* LU, long long lda, int n, T* DinvL, T* DinvU, cudaStream_t st);
+size_t trsv_sync_bytes(int n, int nrhs);
 // X (n x nrhs) <- U^-1 L^-1 X, two persistent launches per pass (FP64:
-// nrhs <= 4; FP32: any nrhs, in passes of 16 beyond 4); `sync` is 4 ints of
-// device scratch.  FP64, and FP32 with `exact`, solve the diagonal blocks by
+// nrhs <= 4; FP32: any nrhs, in passes of 16 beyond 4); `sync` is device scratch of
+// trsv_sync_bytes.  FP64, and FP32 with `exact`, solve the diagonal blocks by
 // substitution; FP32 otherwise multiplies by the block inverses, and corr
 // (two flags per 128-row block: L, U), when given, limits the diagonal-block
 // correction step to flagged blocks.
 // unit_lower = false reads L's stored diagonal (a Cholesky factor G packed
 // with G^T above the diagonal).
-// Bytes of `sync` for n rows and nrhs right-hand sides.
-template <typename T>
-size_t trsv_sync_bytes(int n, int nrhs);
 template <typename T>
 int trsv_lu(const T* LU, long long lda, int n, int nrhs, const T* DinvL, const T* DinvU, T* X, long long ldx,
             void* sync, int* status, cudaStream_t st, const int* corr = nullptr, bool exact = false,
@@ -161,10 +157,6 @@ int nopiv_diag(float* A11, long long lda, int w, int base, float* Lhi, float* Ll
 // 2D copy (rows x cols) between strided buffers on the device.
 template <typename T>
 int copy2d(T* dst, long long ldd, const T* src, long long lds, int rows, int cols, cudaStream_t st);
-
-// Set a rows x cols block to the identity (1 on the diagonal, 0 elsewhere).
-template <typename T>
-int set_identity(T* A, long long lda, int rows, int cols, cudaStream_t st);
 
 // Zero the strict upper triangle of an n x n matrix.
 template <typename T>

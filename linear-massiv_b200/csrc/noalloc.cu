@@ -15,7 +15,9 @@
 
 namespace {
 
-constexpr int kNoAllocMaxN = 4096;  // largest n this entry point accepts
+// Largest n this entry point accepts.  No buffer is sized by it any more; it stays
+// because refusing larger orders is part of the documented interface.
+constexpr int kNoAllocMaxN = 4096;
 
 static __device__ __align__(256) int g_noalloc_status[64];  // [0, 2): error, info
 

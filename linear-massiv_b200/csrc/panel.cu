@@ -59,7 +59,7 @@ struct LeafMsg {
   alignas(16) T v[MW];
 };
 
-template <typename T, int W_, int RPT>
+template <typename T, int W_>
 struct PanelCfg {
   static constexpr int W = W_;
   static constexpr int MW = W < 8 ? W : 8;  // micro-panel width
@@ -262,7 +262,7 @@ template <typename T, int W, int RPT>
 __global__ void __launch_bounds__(kPanelThreads, 1)
     panel_lu_kernel(T* A, long long lda, int n, int c0, int pw, int rpc, unsigned slab_off, int* ipiv, int* plan,
                     int* status) {
-  using Cfg = PanelCfg<T, W, RPT>;
+  using Cfg = PanelCfg<T, W>;
   using Msg = typename Cfg::Msg;
   using Key = typename PivKey<T>::K;
   constexpr int SLD = Cfg::SLD, LDU = Cfg::LDU, MW = Cfg::MW, ZW = Cfg::ZW;
@@ -727,7 +727,7 @@ PanelShape panel_shape(Ctx& c, int rows) {
 template <typename T, int W, int RPT>
 int launch_panel(Ctx& c, const PanelShape& ps, T* A, long long lda, int n, int c0, int pw, int* ipiv, int* plan,
                  cudaStream_t st) {
-  using Cfg = PanelCfg<T, W, RPT>;
+  using Cfg = PanelCfg<T, W>;
   auto kern = panel_lu_kernel<T, W, RPT>;
   static bool attr_set[kMaxDevices] = {};
   const int dev = ctx_device(c);
@@ -762,7 +762,7 @@ int max_cluster(Ctx& c) {
   const int dev = ctx_device(c);
   if (g_max_cluster[dev]) return g_max_cluster[dev];
   int best = 8;
-  using Cfg = PanelCfg<double, 16, 2>;
+  using Cfg = PanelCfg<double, 16>;
   auto kern = panel_lu_kernel<double, 16, 2>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::bytes(kPanelThreads * 2)) ==
           cudaSuccess &&

@@ -3,8 +3,6 @@
 // substitutions rawForwardSubUnitPackedSIMD / rawBackSubPackedSIMD,
 // K.hs:2205-2314).
 //
-//   tri_inv_blocks : inverts every BS x BS diagonal block of L (unit lower)
-//                    and U (upper) once per factorisation;
 //   trsv_kernel    : row-block b (taken in dependency order through an atomic
 //                    ticket, so a block only ever waits on blocks that are
 //                    already running) accumulates  y_b = rhs_b - sum_j T_bj x_j
@@ -14,8 +12,7 @@
 // sentinel (all ones, a NaN) until then, and each thread waits for the entries
 // that it reads.  So one hop through L2 stands between two blocks, where a fence,
 // a progress counter and the load of x after it took three: 5.2 us per 64-row
-// block (FP64) and 6.1 us per 128-row block (FP32) before, 3.1
-// and 3.8 us now.
+// block (FP64) and 6.1 us per 128-row block (FP32) before, 3.1 and 3.8 us now.
 // Each T_bj tile is constant and is loaded before waiting on x_j; the
 // right-hand side and inv(T_bb) are loaded before the first wait.  Every wait
 // is bounded (kSpinLimit polls, then LM_DEVERR_TIMEOUT).
@@ -108,55 +105,6 @@ __device__ __forceinline__ T await(const T* p, int far, bool& ok, int* status) {
   T v;
   memcpy(&v, &u, sizeof v);
   return v;
-}
-
-// inv of the b-th diagonal block of the unit-lower (lower = 1) or upper
-// (lower = 0) factor, row-major BS x BS into Dinv + b * BS * BS.
-template <typename T>
-__global__ void __launch_bounds__(TrsvCfg<T>::NT) tri_inv_blocks_kernel(const T* __restrict__ LU, long long lda,
-                                                                       int n, int lower, T* Dinv) {
-  constexpr int BS = TrsvCfg<T>::BS, NT = TrsvCfg<T>::NT, RG = NT / BS;
-  extern __shared__ __align__(16) unsigned char inv_smem[];
-  T(*Ts)[BS + 1] = reinterpret_cast<T(*)[BS + 1]>(inv_smem);
-  T(*Xs)[BS + 1] = Ts + BS;
-  const int b = blockIdx.x;
-  const int r0 = b * BS;
-  const int w = min(BS, n - r0);
-  for (int i = threadIdx.x; i < BS * BS; i += NT) {
-    const int r = i / BS, c = i % BS;
-    T t = T(0);
-    if (r < w && c < w) {
-      const T v = LU[(long long)(r0 + r) * lda + r0 + c];
-      if (lower)
-        t = (c < r) ? v : (c == r ? T(1) : T(0));
-      else
-        t = (c >= r) ? v : T(0);
-    } else if (r == c) {
-      t = T(1);  // pad the last block with the identity
-    }
-    Ts[r][c] = t;
-    Xs[r][c] = (r == c) ? T(1) : T(0);
-  }
-  __syncthreads();
-  const int c = threadIdx.x % BS;   // column of X this thread updates
-  const int rg = threadIdx.x / BS;  // row group
-  if (lower) {
-    for (int k = 0; k < BS; ++k) {  // rows i > k:  X[i] -= L[i][k] X[k]
-      const T xk = Xs[k][c];
-      for (int i = k + 1 + ((rg - (k + 1)) % RG + RG) % RG; i < BS; i += RG) Xs[i][c] = fma(-Ts[i][k], xk, Xs[i][c]);
-      __syncthreads();
-    }
-  } else {
-    for (int k = BS - 1; k >= 0; --k) {  // X[k] /= U[k][k]; rows i < k: X[i] -= U[i][k] X[k]
-      if (threadIdx.x < BS) Xs[k][threadIdx.x] = Xs[k][threadIdx.x] / Ts[k][k];
-      __syncthreads();
-      const T xk = Xs[k][c];
-      for (int i = rg; i < k; i += RG) Xs[i][c] = fma(-Ts[i][k], xk, Xs[i][c]);
-      __syncthreads();
-    }
-  }
-  T* D = Dinv + (size_t)b * BS * BS;
-  for (int i = threadIdx.x; i < BS * BS; i += NT) D[i] = Xs[i / BS][i % BS];
 }
 
 // Loads this thread's share of a BS-wide slice of row `src` (columns c0 ..):
@@ -469,22 +417,6 @@ size_t trsv_inv_elems(int n) {
   return (size_t)((n + BS - 1) / BS) * BS * BS;
 }
 
-// Inverses of the diagonal blocks of L (unit lower) and U of a packed LU
-// factor: DinvL and DinvU each hold trsv_inv_elems<T>(n) elements.
-template <typename T>
-int tri_inv_blocks(const T* LU, long long lda, int n, T* DinvL, T* DinvU, cudaStream_t st) {
-  constexpr int BS = TrsvCfg<T>::BS, NT = TrsvCfg<T>::NT;
-  if (n <= 0) return LM_OK;
-  const int nb = (n + BS - 1) / BS;
-  const int smem = (int)(2 * BS * (BS + 1) * sizeof(T));
-  LM_CUDA_TRY(cudaFuncSetAttribute(tri_inv_blocks_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  tri_inv_blocks_kernel<T><<<nb, NT, smem, st>>>(LU, lda, n, 1, DinvL);
-  tri_inv_blocks_kernel<T><<<nb, NT, smem, st>>>(LU, lda, n, 0, DinvU);
-  count_launch(2);
-  LM_CUDA_TRY(cudaGetLastError());
-  return LM_OK;
-}
-
 // X (n x nrhs) <- U^-1 L^-1 X with the packed factor (L unit lower, or with
 // its stored diagonal when unit_lower is false, as for a Cholesky factor
 // packed with its transpose).  FP64 and FP32 with `exact` solve the diagonal
@@ -540,14 +472,13 @@ int trsv_lu(const T* LU, long long lda, int n, int nrhs, const T* DinvL, const T
   const int vec_ok = (reinterpret_cast<uintptr_t>(LU) % 16 == 0) && (lda % VEC == 0);
   if (nrhs == 1 && exact)  // the refinement's common case: one column, fewer registers
     return trsv_pass<T, 1, true>(LU, lda, n, nrhs, DinvL, DinvU, X, ldx, sync, status, st, nullptr, vec_ok, ul);
-  if (nrhs <= MAX_RHS) {
-    if (exact)
-      return trsv_pass<T, MAX_RHS, true>(LU, lda, n, nrhs, DinvL, DinvU, X, ldx, sync, status, st, nullptr, vec_ok, ul);
-    return trsv_pass<T, MAX_RHS, false>(LU, lda, n, nrhs, DinvL, DinvU, X, ldx, sync, status, st, corr, vec_ok, ul);
-  }
+  if (nrhs <= MAX_RHS && exact)
+    return trsv_pass<T, MAX_RHS, true>(LU, lda, n, nrhs, DinvL, DinvU, X, ldx, sync, status, st, nullptr, vec_ok, ul);
   if constexpr (kF64) {
     return LM_ERR_UNSUPPORTED;
   } else {
+    if (nrhs <= MAX_RHS)
+      return trsv_pass<T, MAX_RHS, false>(LU, lda, n, nrhs, DinvL, DinvU, X, ldx, sync, status, st, corr, vec_ok, ul);
     // more right-hand sides: the FP32 wide variant, WIDE_RHS columns per pass
     for (int c0 = 0; c0 < nrhs; c0 += WIDE_RHS) {
       const int nc = std::min(WIDE_RHS, nrhs - c0);
@@ -565,9 +496,6 @@ int trsv_lu(const T* LU, long long lda, int n, int nrhs, const T* DinvL, const T
 template size_t trsv_sync_bytes<float>(int, int);
 template size_t trsv_sync_bytes<double>(int, int);
 template size_t trsv_inv_elems<float>(int);
-template size_t trsv_inv_elems<double>(int);
-template int tri_inv_blocks<float>(const float*, long long, int, float*, float*, cudaStream_t);
-template int tri_inv_blocks<double>(const double*, long long, int, double*, double*, cudaStream_t);
 template int trsv_lu<float>(const float*, long long, int, int, const float*, const float*, float*, long long, void*,
                             int*, cudaStream_t, const int*, bool, bool);
 template int trsv_lu<double>(const double*, long long, int, int, const double*, const double*, double*, long long,
