@@ -159,8 +159,9 @@ int lm_ipiv_to_perm(int n, const int* ipiv, int* perm);
 
 /* ---- mixed precision with iterative refinement -----------------------------
  * No counterpart in the reference (its solves are FP64 throughout).  A is
- * rounded to FP32 and factored with partial pivoting, every Schur-complement
- * update on the tcgen05 tensor cores in TF32 with FP32 accumulation; the
+ * rounded to FP32 and factored with partial pivoting, the updates right of a
+ * 128-column panel on the tcgen05 tensor cores in TF32 with FP32 accumulation,
+ * those inside it as FP32 multiply-adds; the
  * solution is then refined in FP64 (residual r = B - A X with the original A,
  * correction from the FP32 factors, X += d) until the normwise backward error
  * ||r||_inf / (||A||_inf ||x||_inf + ||b||_inf) of every column is <= tol
@@ -177,8 +178,8 @@ int lm_lu_solve_ir_host(lm_ctx* ctx, int n, int nrhs, const double* A, const dou
 /* Factorisation used by the mixed-precision solves of a context (lm_dgesv_ir,
  * lm_lu_solve_ir_host and the serving loop's large requests).
  *   LM_IR_GEPP (default): FP32 LU with partial pivoting (the FP64 path's pivot
- *     rule), every Schur-complement update as 3xTF32 on the tensor cores, with
- *     look-ahead; the FP32 substitutions solve their diagonal blocks by
+ *     rule), the updates right of a panel as 3xTF32 on the tensor cores (inside it
+ *     FP32 multiply-adds), with look-ahead; the FP32 substitutions solve their diagonal blocks by
  *     substitution, so each correction is backward stable in FP32.
  *   LM_IR_RBT: A is mixed by two random depth-2 butterfly transforms,
  *     Ar = U^T A V (Baboulin, Dongarra, Herrmann, Tomov 2013), and Ar is
@@ -233,7 +234,7 @@ int lm_ctx_ir_history(lm_ctx* ctx, double* berr, int max_steps, int* steps);
  * the first call on that device looks up its address (CUDA loads device code
  * lazily by default) and held until exit: make that first call (n = 0 does
  * only this) before any region that must not allocate and before any stream
- * capture.  n is limited to 4096 (larger n returns LM_ERR_ARG) and A must be
+ * capture.  n is limited to 4096 by contract (larger n returns LM_ERR_ARG) and A must be
  * 16-byte aligned with an even lda.  All calls share the status words: calls
  * that overlap on the GPU race and must be serialised by the caller. */
 int lm_dpotrf_noalloc(void* stream, int n, double* A, int lda, int* info);
