@@ -708,7 +708,7 @@ def run_reference(a, world, rank):
 # run's per-launch traffic is this ratio times its own algorithmic bytes per
 # launch (the traffic of these launches grows in proportion to their size).
 DRAM_PER_ALGO_BYTE = {
-    "dgemm": 1.11e9 / 1.090e9,
+    "dgemm": 1.057e9 / 1.090e9,
     "sgemm": 481.2e6 / 528.0e6,
 }
 

@@ -18,11 +18,12 @@
 // main loop runs, so the epilogue reads C on chip instead of waiting on
 // L2/HBM.  The CTAs of an SM drift apart, so that one's epilogue and first loads
 // run under the others' DMMAs, and small tiles leave less of the last wave idle.
-// Against 128 x 128 tiles with one CTA per SM (before):
-//   k = 128, beta = 1 : m = n = 8192 591 -> 579 us, 16384 2316 -> 2271 us,
-//                       8192 x 128 24.9 -> 15.5 us, 8192 x 64 22.8 -> 11.5 us;
-//   square            : 500 80 -> 27 us, 1000 150 -> 76 us, 2000 (1500 x 1002)
-//                       289 -> 226 us, 4096 4.05 -> 3.94 ms, 8192 32.1 -> 31.2 ms.
+// Against 128 x 128 tiles with one CTA per SM (before, and without the wait of
+// give_back, which costs 2 to 3%):
+//   k = 128, beta = 1 : m = n = 8192 591 -> 598 us, 16384 2316 -> 2346 us,
+//                       8192 x 128 24.9 -> 16.6 us, 8192 x 64 22.8 -> 12.9 us;
+//   square            : 500 80 -> 30 us, 1000 150 -> 78 us, 2000 (1500 x 1002)
+//                       289 -> 239 us, 4096 4.05 -> 4.04 ms, 8192 32.1 -> 32.0 ms.
 // Tiles go to CTAs by index, or, for a product that runs beside other kernels (the
 // trailing updates beside a panel), by tickets: CTAs that find their SM taken start
 // when it is free and take what is left, and SMs can be kept clear for a kernel
@@ -487,8 +488,8 @@ int dgemm(Ctx& ctx, const GemmDesc& d, cudaStream_t st) {
   // Short k with beta != 0 (the factorisations' trailing updates): C staged in
   // shared memory, three CTAs per SM with two k-slices each in flight.  Beyond
   // k = 256 the C traffic no longer counts and a deeper ring does: two CTAs per SM
-  // (4096^3: 3.97 ms, and 4.18 ms with three; k = 128, m = n = 4000: 0.195 ms with
-  // two and 0.147 ms with three).
+  // (before the wait of give_back: 4096^3 3.97 ms, and 4.18 ms with three; k = 128,
+  // m = n = 4000 0.195 ms with two and 0.147 ms with three, 0.153 ms now).
   const double flops = d.lower_only ? (double)d.m * (d.m + 1) * d.k : 2.0 * d.m * d.n * d.k;
   const double bytes = 8.0 * ((double)d.m * d.k + (double)d.k * d.n +
                               (d.beta != 0.0 ? 2.0 : 1.0) * (d.lower_only ? 0.5 : 1.0) * d.m * d.n);

@@ -23,8 +23,9 @@
 //   (with the reciprocal of the leading entry, formed while the warp votes)
 //   are all that a candidate sends, and the rest of the leaf's columns is
 //   updated once per micro-panel with the 8 pivot rows, which their owners
-//   send on the side.  What bounds a column is instruction latency: about 250
-//   instructions at 6 to 7 cycles with one to four warps per scheduler.
+//   send on the side.  What bounds a column is instruction latency: about 480
+//   instructions per warp, with the solves and updates, at 7.4 cycles each and one
+//   to four warps per scheduler.
 //   A 128-column panel takes 205 us at 500 to 2000 rows (FP64); the 32-column
 //   leaves before it took 63 us each, with 100 us of small solves, products
 //   and interchanges between the four of them (8192 rows).
